@@ -33,6 +33,7 @@ Sweep2Launch make_launch(const elp_group* G, int nsteps, uint32_t step_base, int
     l.args.step_base = step_base;
     l.args.step_dev = G->d_ctr;
     l.args.table = G->d_table;
+    l.args.moves = G->d_moves;
     l.args.error = G->d_error;
     l.args.grid_bar = G->d_ctr + 1;
     l.args.wait_polls = G->wait_polls;
@@ -98,7 +99,12 @@ cudaError_t elp_group_init(elp_group* G, const elp_geometry& geom, int nsm, int 
     // stream-ordered (a group created while others run does not stall them)
     cudaError_t e = cudaMallocAsync((void**)&G->d_ctr, 4 * sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
-    return cudaMemsetAsync(G->d_ctr, 0, 4 * sizeof(uint32_t), stream);
+    if ((e = cudaMemsetAsync(G->d_ctr, 0, 4 * sizeof(uint32_t), stream)) != cudaSuccess) return e;
+    uint32_t moves[ELP_MOVES_MAX];
+    const int n = elp_move_table(&geom, &G->lay, moves);
+    if ((e = cudaMallocAsync((void**)&G->d_moves, sizeof(moves), stream)) != cudaSuccess) return e;
+    // pageable source: the call returns once the words are staged
+    return cudaMemcpyAsync(G->d_moves, moves, (size_t)n * sizeof(uint32_t), cudaMemcpyHostToDevice, stream);
 }
 
 void elp_group_add(elp_group* G, uint32_t* lat, uint32_t* rec, unsigned long long* acc, int N, int nchains,
@@ -240,9 +246,11 @@ void elp_group_free(elp_group* G)
     if (G->stream) cudaStreamSynchronize(G->stream);
     cudaFree(G->d_jobs);
     cudaFree(G->d_items);
+    cudaFree(G->d_moves);
     cudaFree(G->d_ctr);
     G->graph = nullptr;
     G->d_jobs = nullptr;
     G->d_items = nullptr;
+    G->d_moves = nullptr;
     G->d_ctr = nullptr;
 }

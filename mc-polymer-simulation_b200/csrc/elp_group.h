@@ -34,6 +34,7 @@ struct elp_group {
     uint2* d_items = nullptr;
     int nitems = 0;
     size_t cap_jobs = 0, cap_items = 0;   // grow-only device capacity of the two tables
+    uint32_t* d_moves = nullptr;      // move table and neighbour offsets (elp_move_table)
     uint32_t* d_ctr = nullptr;        // device step counter, then the grid barrier's two counts
     uint32_t wait_polls = 0;          // bound of the grid barrier's waits (0: the kernel's default)
     int hold_cta1 = 0;                // test hook: CTA + 1 that never arrives at the first barrier

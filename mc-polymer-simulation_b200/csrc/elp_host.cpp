@@ -234,6 +234,61 @@ void elp_build_table(uint8_t tab[4096])
     for (int i = 0; i < 4096; i++) tab[i] = (uint8_t)(T.e[i] & 0xff);
 }
 
+// Tables of the specialised sweep kernels (elp_sweep2.cu), in the order they
+// are copied to shared memory.  Returns the number of words.
+//
+// Move table: entry (s1 << 8 | s2 << 4 | r) for option r = d1 | d2 << 4 of
+// row (s1, s2) of the transition table, 0 for no move:
+//   bits 0-4    test: a target word with one of these bits set rejects the
+//               move (a new site must be empty: every code bit and the wall
+//               bit; a run to join must not be a wall; joining the anchor's
+//               own run: no test).  Whole boxes have no walls.
+//   bits 5-8    the anchor's new b_out
+//   bits 9-12   d2, the new site's b_out (0: none)
+//   bits 16-17  change of the anchor's run length, plus 1
+//   bits 18-31  tiles: byte offset of the target, signed (bits 18, 19 zero)
+//   bits 28-31  whole box: d1, an index into the boundary class's offsets
+// Empty besides: rows whose source is no bond (3, 12: wall words).
+//
+// Neighbour offsets: for each code b {word offset << 16 | row of b << 10},
+// the row an empty one (3) for b = 0xf (slot 1 at the last run of a linear
+// chain, which has no next run), for the 27 boundary classes (cx + 3 cy + 9 cz; 0 first plane, 1 inside, 2 last) of
+// a whole box, else once, followed by the plain word offsets.
+int elp_move_table(const elp_geometry* g, const elp_smem_layout* lay, uint32_t out[ELP_MOVES_MAX])
+{
+    uint8_t tab[4096];
+    elp_build_table(tab);
+    const int sx = lay->sx, sxy = lay->sxy;
+    for (uint32_t i = 0; i < ELP_MOVE_ENTRIES; i++) {
+        const uint32_t s1 = i >> 8, s2 = (i >> 4) & 15, e = tab[i], d1 = e & 15, d2 = e >> 4;
+        out[i] = 0;
+        if (!e || s1 == 3 || s1 == 12 || s2 == 3 || s2 == 12) continue;
+        const uint32_t test = !d2 ? 0x10u : (d1 ? 0x1Fu : 0u);
+        const uint32_t dcnt = s1 == 0 ? 0u : (d1 ? 1u : 2u);
+        const int off = 4 * (elp_bt(d1) + sx * elp_bu(d1) + sxy * elp_bv(d1));
+        out[i] = (g->periodic ? (test & 15u) | (d1 << 28) : test | ((uint32_t)off << 18)) | ((d1 ? d1 : d2) << 5) |
+                 (d2 << 9) | (dcnt << 16);
+    }
+    int n = ELP_MOVE_ENTRIES;
+    for (int cls = 0; cls < (g->periodic ? 27 : 1); cls++)
+        for (uint32_t b = 0; b < 16; b++) {
+            int dt = elp_bt(b), du = elp_bu(b), dv = elp_bv(b);
+            if (g->periodic) {
+                const int cx = cls % 3, cy = (cls / 3) % 3, cz = cls / 9, wrap = g->L - 1;
+                if (cx == 0 && dt < 0) dt = wrap;
+                if (cx == 2 && dt > 0) dt = -wrap;
+                if (cy == 0 && du < 0) du = wrap;
+                if (cy == 2 && du > 0) du = -wrap;
+                if (cz == 0 && dv < 0) dv = wrap;
+                if (cz == 2 && dv > 0) dv = -wrap;
+            }
+            out[n++] = ((uint32_t)(dt + sx * du + sxy * dv) << 16) | ((b == 15 ? 3u : b) << 10);
+        }
+    if (!g->periodic)
+        for (uint32_t b = 0; b < 16; b++) out[n++] = (uint32_t)(elp_bt(b) + sx * elp_bu(b) + sxy * elp_bv(b));
+    return n;
+}
+
 // Time factors of tiled geometries: eight GPU melts of N=100 rings (density
 // 1.2) against the eight reference efpol melts at L=64, the centre-of-mass
 // MSD over steps 15000-50000 at lags of 500 to 25000 steps; f is the step

@@ -8,8 +8,9 @@
 //   label set:   bits 5-31 chain id; the run length is in the chain record
 //   0          empty site
 // (Inside the specialised sweep kernels a labelled word is rewritten while its
-// tile is on chip: bits 5-15 index a shared-memory label slot and bits 16-31
-// hold the run length, so every on-chip word carries its count.)
+// tile is on chip: bits 5-15, 4-15 in a whole box, hold the number of a
+// shared-memory label slot plus 1 and bits 16-31 the run length, so every
+// on-chip word carries its count.)
 // Chain record (4 x uint32 per chain): {global site of monomer 0's run,
 //   length of that run, offset of monomer 0 inside it, unused}.
 //
@@ -68,6 +69,11 @@ int elp_geometry_ok(const elp_geometry* g);
 void elp_layout(const elp_geometry* g, elp_smem_layout* lay);
 void elp_philox_host(const uint32_t ctr[4], const uint32_t key[2], uint32_t out[4]);
 void elp_build_table(uint8_t tab[4096]);
+// Move table (rows s1 = 0 .. 14), neighbour offsets (27 * 16 words for a
+// whole box, 16 + 16 for tiles) of the specialised kernels.
+#define ELP_MOVE_ENTRIES (15 * 256)
+#define ELP_MOVES_MAX (ELP_MOVE_ENTRIES + 27 * 16)
+int elp_move_table(const elp_geometry* g, const elp_smem_layout* lay, uint32_t out[ELP_MOVES_MAX]);
 int elp_get_npol(double density, int N, long sites);
 // The grid of CreatePolymers (cpupol/efpol_init.c:239-283): chain p starts at
 // (delta (p % nt), delta (p / nt / nv), (delta + 1) ((p / nt) % nv)).

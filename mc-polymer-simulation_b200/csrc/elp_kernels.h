@@ -50,6 +50,7 @@ struct BatchLaunch {
     uint32_t step_base;            // added to every job's step0 ...
     const uint32_t* step_dev;      // ... and, if set, this device counter (graph replays)
     const uint32_t* table;         // 4096-byte transition table
+    const uint32_t* moves;         // move table and neighbour offsets of the geometry (elp_move_table)
     uint32_t* error;               // device error flags (bit 0: label slot table overflow,
                                    // bit 2: a grid barrier wait gave up)
     uint32_t* grid_bar;            // tiled domains, nsteps > 1: {arrivals, exits}, zero between launches

@@ -6,23 +6,22 @@
 //   * the K anchors a thread owns in a substep are processed stage by stage
 //     (all first loads, then all second loads, ...), so the dependent
 //     shared-memory loads of independent moves overlap;
-//   * monomer 0's runs are handled inline: while a tile is on chip each
-//     labelled word carries its run length (bits 16-31) and a slot number
-//     (bits 5-15) into a small shared-memory table {chain, offset | site};
-//     the chain records in global memory are read when the tile is loaded and
+//   * monomer 0's runs are handled inline: while a domain is on chip each
+//     labelled word carries its run length (bits 16-31) and the number of a
+//     slot of a small shared-memory table {chain, offset of monomer 0}; the
+//     chain records in global memory are read when the domain is loaded and
 //     written back when it is stored, so no move waits on global memory.  A
 //     ring tile that holds more monomer-0 runs than the table (short rings
 //     crowded together, as CreatePolymers leaves them) runs its substeps with
 //     the general move of elp_device.cuh instead, which keeps that
 //     bookkeeping in the chain records: slower, the same bits;
-//   * a tile's rows are fetched in 16-byte cp.async granules.  The origin
-//     shift makes a row start anywhere, so each row fetch takes the 16-byte
-//     aligned span around the row (TX + 4 words) and the tile sits
-//     sh = x0 mod 4 words into it; the words of the span outside the tile
-//     become halo words.  Tiles go back with 16-byte stores (single words at
-//     the ragged ends).  Rows are 16-byte aligned in shared memory, and the
-//     threads of a warp take anchors from an 8 x 4 block of rows so that
-//     their first loads hit 32 different banks;
+//   * a tile's rows move in 16-byte words.  The origin shift makes a row
+//     start anywhere, so each row fetch takes the 16-byte aligned span around
+//     the row (TX + 4 words) and the tile sits sh = x0 mod 4 words into it;
+//     the words of the span outside the tile become halo words.  Rows are
+//     16-byte aligned in shared memory, and the threads of a warp take
+//     anchors from an 8 x 4 block of rows so that their first loads hit 32
+//     different banks;
 //   * the grid is persistent over the tiles, and a launch of several steps
 //     over a tiled box is cooperative, with a grid barrier between steps.
 #include <cuda_runtime.h>
@@ -35,11 +34,6 @@
 
 namespace elp {
 
-__device__ __forceinline__ void cp_async4(uint32_t* sdst, const uint32_t* gsrc)
-{
-    uint32_t s = (uint32_t)__cvta_generic_to_shared(sdst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gsrc) : "memory");
-}
 __device__ __forceinline__ void cp_async16(uint32_t* sdst, const uint32_t* gsrc)
 {
     uint32_t s = (uint32_t)__cvta_generic_to_shared(sdst);
@@ -57,22 +51,23 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p)
 // back-off below); a launch can ask for fewer (BatchLaunch.wait_polls).
 constexpr uint32_t WAIT_POLLS = 1u << 24;
 
-// Barrier over all CTAs of a cooperative launch: each CTA adds one to
-// bar[0] and waits (bounded) until it reaches `target`.  The CTA's stores
-// before it are visible to every CTA's loads after it (tiles are fetched
-// with cp.async.cg and records with ld.global.cg, both through L2).
+// Barrier over all CTAs of a cooperative launch, in two halves: each CTA adds
+// one to bar[0] (its stores before that are visible to every CTA's loads
+// after the wait: tiles and records are loaded with ld.global.cg, through L2)
+// and later waits (bounded) until the count reaches `target`.
+__device__ __forceinline__ void grid_arrive(uint32_t* bar)
+{
+    __threadfence();
+    atomicAdd(bar, 1u);
+}
 // Returns false, in every thread of the CTA, when the wait gave up.
-// `arrive` false (a test) makes the CTA wait without adding its count.
-__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t target, uint32_t polls, bool arrive)
+__device__ __forceinline__ bool grid_wait(uint32_t* bar, uint32_t target, uint32_t polls)
 {
     bool ok = true;
-    __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        if (arrive) atomicAdd(bar, 1u);
         for (uint32_t n = 0; ld_acquire_gpu(bar) < target; n++) {
             if (n >= polls) { ok = false; break; }
-            __nanosleep(64);
+            __nanosleep(32);
         }
     }
     return __syncthreads_or(!ok) == 0;
@@ -94,122 +89,303 @@ struct Shape {
     static constexpr int A = R * (TX / NC);   // anchors per substep
     static constexpr int G = A / 4;           // Philox counters per substep group
     static constexpr int AT = A / K;          // threads that own anchors
+    static constexpr int THREADS = (AT + 31) / 32 * 32;
+    static constexpr bool TAIL = AT != THREADS;   // threads without anchors fill the last warp
     // Tiled domains: row y of plane z starts at OX + SX y + SXY z (16-byte
     // aligned) and holds the copied span of TX + 4 words, the tile at offset
     // sh in it; rows y = -1, TY and planes z = -1, TZ are halo, as is the
     // word before each row (the previous row's padding).
     static constexpr int SPAN = TX + 4;
     static constexpr int OX = PER ? 0 : SX + SXY + 4;
-    static constexpr int WORDS = PER ? SXY * TZ : ((OX + SX * TY + SXY * TZ + SPAN + 3) & ~3);
-    static constexpr int SITES = TX * TY * TZ;
+    static constexpr int WORDS = PER ? (SXY * TZ + 3) & ~3 : ((OX + SX * TY + SXY * TZ + SPAN + 3) & ~3);
+    // A tile moves in NP passes: thread tid < AT takes word quad tid % CB of
+    // row tid / CB, ZS planes further on each pass; the quad at the row's end
+    // (held words if sh > 0) is one more pass over the rows.
+    static constexpr int CB = TX / 4;
+    static constexpr int NP = R * CB / AT;
+    static constexpr int ZS = TZ / NP > 0 ? TZ / NP : 1;
     // threads of a warp take anchors from an 8 x 4 block of (y, z) rows
     static constexpr bool PERM = !PER && TY % 8 == 0 && TZ % 4 == 0 && AT % R == 0;
     // neighbour offsets: 27 boundary classes of a periodic box, one class in a tile
     static constexpr int NOFF = PER ? 27 * 16 : 16;
-    // shared-memory word offsets: lattice, transition table (4096 bytes),
-    // neighbour offsets (bytes, and for tiles in words too), colours, slot
-    // tables, slot count, head-move rows, and the Philox words when threads
-    // own < 4 anchors
+    // a labelled on-chip word holds its slot number + 1 above bit LSH (a
+    // tile's bit 4 marks walls, a whole box has none)
+    static constexpr int LSH = PER ? 4 : 5;
+    static constexpr uint32_t LMASK = 0xFFFFu & ~((1u << LSH) - 1u);
+    static constexpr int SLOTS = CAP < (int)(LMASK >> LSH) ? CAP : (int)(LMASK >> LSH);
+    // shared-memory word offsets: lattice, move table, neighbour
+    // offsets (tiles: plain word offsets too, for the general move), colours,
+    // slot table (chain, offset of monomer 0 in its run), head-move rows,
+    // random bytes
     static constexpr int TABW = WORDS;
-    static constexpr int OFFW = TABW + 1024;
+    static constexpr int OFFW = TABW + ELP_MOVE_ENTRIES;
     static constexpr int WOFFW = OFFW + NOFF;
-    static constexpr int COLW = WOFFW + (PER ? 0 : 16);
-    static constexpr int SHFW = COLW + 64;    // the step's domain shift (tiles), drawn by one warp
-    static constexpr int SCHW = SHFW + 4;
-    static constexpr int SSOW = SCHW + CAP;   // {offset of monomer 0 in its run (bits 0-15), site word (16-31)}
-    static constexpr int NSLW = SSOW + CAP;
-    static constexpr int HTABW = NSLW + 1;    // table rows (0xf, x): moves of a linear chain's monomer 0
+    static constexpr int COLW = (WOFFW + (PER ? 0 : 16) + 3) & ~3;
+    static constexpr int NSLW = COLW + 4 * ((2 * NC + 3) / 4);   // slot count
+    static constexpr int TILEW = (NSLW + 4) & ~3;                // the tile at hand (Tile)
+    static constexpr int SCHW = TILEW + 16;
+    static constexpr int SLOW = SCHW + CAP;
+    static constexpr int HTABW = SLOW + CAP;  // table rows (0xf, x): moves of a linear chain's monomer 0
     static constexpr int RNDW = (HTABW + 64 + 3) & ~3;
-    static constexpr int NG = 2 * NC / 4;     // substep groups per step
-    static constexpr size_t bytes_with(int groups) { return (size_t)(RNDW + (K < 4 ? groups * G * 4 : 0)) * 4; }
-    // Philox words of threads that own < 4 anchors: in tiled domains, where
-    // MINB CTAs still fit on an SM (228 KB, 1 KB reserved per CTA), all NG
-    // groups of the step, drawn while the tile loads (PRE); else two buffers,
-    // the next group's drawn during this one
-    static constexpr bool PRE = !PER && K < 4 && (size_t)MINB * (bytes_with(NG) + 1024) <= 233472;
-    static constexpr int TOTW = RNDW + (K < 4 ? (PRE ? NG : 2) * G * 4 : 0);
+    static constexpr int NSUB = 2 * NC;              // substeps per step
+    static constexpr int NG = (NSUB + 3) / 4;        // groups of four substeps
+    // Random bytes, 16 per counter and group: in tiled domains, where MINB
+    // CTAs still fit on an SM (228 KB, 1 KB reserved per CTA), all NG groups
+    // of the step, drawn before its substeps (PRE); else one group's, read
+    // into registers as the group starts and overwritten with the next
+    // group's after its first barrier
+    static constexpr size_t bytes_with(int groups) { return (size_t)(RNDW + groups * A) * 4; }
+    static constexpr bool PRE = !PER && (size_t)MINB * (bytes_with(NG) + 1024) <= 233472;
+    static constexpr int TOTW = RNDW + (PRE ? NG : 1) * A;
     static constexpr size_t BYTES = (size_t)TOTW * 4;
+    // neighbour offsets in words fit 16 signed bits (else they are taken
+    // modulo 2^16, the reach of a shared-memory word index)
+    static constexpr bool SOFF = !PER || (TX - 1) * (1 + SX + SXY) <= 32767;
+    static_assert(A % 4 == 0 && A % K == 0 && THREADS <= 1024 && G <= THREADS, "anchors and draws per thread");
+    static_assert(K == 1 || (K == 2 && (A / 2) % G == 0), "the anchors of a thread share a Philox counter");
+    static_assert(CAP <= 2048, "slot numbers");
     static_assert(PER || (SX % 4 == 0 && SXY % 4 == 0 && SX >= SPAN + 1 && SXY >= SX * (TY + 2)),
                   "tiled rows: 16-byte aligned, room for the span and the halo word before it");
+    static_assert(PER || (NP * AT == R * CB && AT % (CB * TY) == 0 && TZ % NP == 0 && R <= AT && TX % 4 == 0),
+                  "a pass of the tile copy takes whole planes");
     static_assert(WORDS < 65536, "slot sites are 16-bit word indices");
     static_assert(BYTES <= 232448, "dynamic shared memory of one CTA");
 };
 
-constexpr uint32_t LMASK = 0xFFF0u;  // label bit + slot number
-// Halo word of tiled domains: run length 1, b_out 3 (not a bond).  A slot-1
-// move whose next run lies in the halo then looks up row (b_out(P), 3) of
-// the table, which the kernel clears in its shared-memory copy, so the move
-// is null without a separate test; a target in the halo is neither empty nor
-// a run of the chain, so it is rejected as well.
-constexpr uint32_t HWALL = ELP_CUNIT | 3u;
+// Halo word of tiled domains: bit 4 (no other on-chip word has it), run
+// length 1, b_out 3 (not a bond).  A slot-1 move whose next run lies in the
+// halo looks up row (b_out(P), 3) of the move table, which is empty; a target
+// in the halo meets the entry's test bits (bit 4 among them for moves onto a
+// site or a run).
+constexpr uint32_t HWALL = ELP_CUNIT | 0x10u | 3u;
 
 extern __shared__ __align__(16) uint32_t g_smem[];
-
-// A labelled word (global form: chain id in bits 5-31) entering shared
-// memory: claim a slot for the chain, keep {chain, offset | site} in the
-// slot table and put the slot number and the run length into the word.  Past
-// the table's capacity the word is left as it is (the tile then runs the
-// general move).
-template <int CAP>
-__device__ __forceinline__ uint32_t take_slot(uint32_t wv, int idx, const uint32_t* rec, uint32_t* nslots,
-                                              uint32_t* slot_chain, uint32_t* slot_so)
-{
-    const uint32_t slot = atomicAdd(nslots, 1u);
-    if (slot >= (uint32_t)CAP) return wv;
-    const uint32_t chain = wv >> 5;
-    const uint4 rr = __ldcg(reinterpret_cast<const uint4*>(rec + ELP_REC_WORDS * (size_t)chain));
-    slot_chain[slot] = chain;
-    slot_so[slot] = rr.z | ((uint32_t)idx << 16);
-    return (wv & 15) | ELP_LBIT | (slot << 5) | (rr.y << ELP_CSHIFT);
-}
 
 // Shared-memory word at byte offset b (offsets are kept in bytes so that a
 // load or store needs no index scaling).
 __device__ __forceinline__ uint32_t& SW(int b) { return *reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(g_smem) + b); }
 
-// Monomer 0 sits in one of the runs a move touches (src: 0 the anchor's run,
-// 1 the next run, 2 the target run): move its slot's site and offset along.
-// Updates the new word (nP, nB or nY) that ends up holding monomer 0.
-__device__ __forceinline__ void follow_label(uint32_t* slot_so, int p, int pB, int pY, uint32_t wP, uint32_t wB,
-                                             uint32_t wY, uint32_t s, uint32_t d1, uint32_t& nP, uint32_t& nB,
-                                             uint32_t& nY)
+// A labelled word (global form: chain id in bits 5-31) has come into shared
+// memory at word idx: claim a slot for its chain.  Past the table's capacity
+// it is only counted.
+template <class SH>
+__device__ __forceinline__ void claim_slot(uint32_t wv, int idx)
 {
-    const int src = (wP & ELP_LBIT) ? 0 : ((s && (wB & ELP_LBIT)) ? 1 : 2);
-    const uint32_t lw = src == 0 ? wP : (src == 1 ? wB : wY);
-    const uint32_t slot = (lw >> 5) & 0x7FFu;
-    const uint32_t off0 = slot_so[slot] & 0xFFFFu;
-    uint32_t noff;
-    int nl;
-    if (src == 0) {
-        nl = 0; noff = off0;
-        if (s == 0 && off0 == (wP >> ELP_CSHIFT) - 1) { nl = 2; noff = 0; }
-    } else if (src == 1) {
-        if (wB >= 2u * ELP_CUNIT && off0 > 0) { nl = 1; noff = off0 - 1; }
-        else { nl = d1 ? 2 : 0; noff = d1 ? 0 : (nP >> ELP_CSHIFT) - 1; }
-    } else {
-        nl = 2; noff = off0 + 1;
+    const uint32_t slot = atomicAdd(g_smem + SH::NSLW, 1u);
+    if (slot >= (uint32_t)SH::SLOTS) return;
+    g_smem[SH::SCHW + slot] = wv >> 5;
+    g_smem[SH::SLOW + slot] = (uint32_t)idx;   // until the record is fetched
+}
+// Fetch the chain record of each claimed slot: the word gets the slot number
+// and the run length, the slot monomer 0's offset.
+template <class SH>
+__device__ __forceinline__ void fill_slots(const uint32_t* rec, uint32_t ns)
+{
+    for (uint32_t sl = threadIdx.x; sl < ns; sl += SH::THREADS) {
+        const uint32_t idx = g_smem[SH::SLOW + sl];
+        const uint4 rr = __ldcg(reinterpret_cast<const uint4*>(rec + ELP_REC_WORDS * (size_t)g_smem[SH::SCHW + sl]));
+        g_smem[idx] = (g_smem[idx] & 15) | ((sl + 1) << SH::LSH) | (rr.y << ELP_CSHIFT);
+        g_smem[SH::SLOW + sl] = rr.z;
     }
-    const uint32_t lb = lw & LMASK;
-    if (src == 0) nP &= ~LMASK; else if (src == 1) nB &= ~LMASK; else nY &= ~LMASK;
-    if (nl == 0) nP |= lb; else if (nl == 1) nB |= lb; else nY |= lb;
-    slot_so[slot] = noff | ((uint32_t)((nl == 0 ? p : (nl == 1 ? pB : pY)) >> 2) << 16);
+}
+// A labelled word on its way out, from box site `site`: write the chain's
+// record and return the word's global form.
+template <class SH>
+__device__ __forceinline__ uint32_t leave_slot(uint32_t wv, uint32_t site, uint32_t* rec)
+{
+    const uint32_t slot = ((wv & SH::LMASK) >> SH::LSH) - 1u;
+    const uint32_t chain = g_smem[SH::SCHW + slot];
+    *reinterpret_cast<uint4*>(rec + ELP_REC_WORDS * (size_t)chain) =
+        make_uint4(site, wv >> ELP_CSHIFT, g_smem[SH::SLOW + slot], 0u);
+    return (wv & 15) | ELP_LBIT | (chain << 5);
 }
 
-// The Philox word of substep group k / 4 for this thread's anchors (counter
-// word 3 gq).  Threads owning four anchors draw it themselves; with PRE all
-// of the step's words were drawn while the tile loaded; otherwise G threads
-// draw the next group's words into the other of two buffers while this group
-// runs (read four barriers ago).
-template <int K, bool PRE, int G, int NSUB>
-__device__ __forceinline__ uint4 group_words(uint4* rnd, int k, uint32_t t, int d, int gq, uint2 key)
+// Monomer 0 sits in one of the runs an accepted move touched, whose new words
+// nP, nB, nY are stored (each with the label bits its old word had): bring its
+// slot number and offset to the run that holds it now.  Rarely needed; the
+// volatile accesses keep the compiler from folding it into the common case's
+// stores as selects that every move would pay for.
+template <class SH>
+__device__ __forceinline__ void follow_label(int p, int pB, int pY, uint32_t wP, uint32_t wB, uint32_t wY, bool s,
+                                             bool d1, bool join, uint32_t nP, uint32_t nB, uint32_t nY)
 {
-    if (K == 4) return philox(make_uint4(t, (uint32_t)d, (uint32_t)(k >> 2), (uint32_t)gq), key);
-    if (PRE) return rnd[(k >> 2) * G + gq];
-    const int cur = (k >> 2) & 1;
-    const uint4 rw = rnd[cur * G + gq];
-    if ((int)threadIdx.x < G && k + 4 < NSUB)
-        rnd[(cur ^ 1) * G + threadIdx.x] = philox(make_uint4(t, (uint32_t)d, (uint32_t)(k >> 2) + 1u, threadIdx.x), key);
-    return rw;
+    constexpr uint32_t LMASK = SH::LMASK;
+    volatile uint32_t* const slot_off = g_smem + SH::SLOW - 1;
+    volatile char* const S = reinterpret_cast<volatile char*>(g_smem);
+    auto put = [&](int b, uint32_t w) { *reinterpret_cast<volatile uint32_t*>(S + b) = w; };
+    if (wP & LMASK) {
+        // the anchor's run: monomer 0 leaves it as its last monomer only
+        const uint32_t lb = wP & LMASK;
+        if (!s && slot_off[lb >> SH::LSH] == (wP >> ELP_CSHIFT) - 1) {
+            put(p, nP & ~LMASK);
+            put(pY, nY | lb);
+            slot_off[lb >> SH::LSH] = 0;
+        }
+    } else if (s && (wB & LMASK)) {
+        // the next run, whose first monomer moves: monomer 0 stays (one place
+        // nearer the front) unless it is that monomer
+        const uint32_t lb = wB & LMASK, off0 = slot_off[lb >> SH::LSH];
+        if (off0 > 0) {
+            slot_off[lb >> SH::LSH] = off0 - 1;
+        } else {
+            put(pB, nB & ~LMASK);
+            if (d1) put(pY, nY | lb);
+            else put(p, nP | lb);
+            slot_off[lb >> SH::LSH] = d1 ? 0u : (nP >> ELP_CSHIFT) - 1;
+        }
+    } else if (join && (wY & LMASK)) {
+        const uint32_t sl = (wY & LMASK) >> SH::LSH;   // a monomer joins its front
+        slot_off[sl] = slot_off[sl] + 1;
+    }
+}
+
+// Random bytes of one substep group: byte q of words 0-3 of Philox counter
+// {t, d, group, gq} serves anchor gq + q G in the group's four substeps: bit
+// 0 the slot s, bits 1-4 the table option.  Kept with s in bit 7 and the
+// option in bits 2-5 of its byte: the slot then spreads over a byte by sign
+// replication and the option is a word offset.
+__device__ __forceinline__ uint4 draw_bytes(uint32_t t, int d, int group, int gq, uint2 key)
+{
+    uint4 v = philox(make_uint4(t, (uint32_t)d, (uint32_t)group, (uint32_t)gq), key);
+    v.x = ((v.x << 7) & 0x80808080u) | ((v.x << 1) & 0x3C3C3C3Cu);
+    v.y = ((v.y << 7) & 0x80808080u) | ((v.y << 1) & 0x3C3C3C3Cu);
+    v.z = ((v.z << 7) & 0x80808080u) | ((v.z << 1) & 0x3C3C3C3Cu);
+    v.w = ((v.w << 7) & 0x80808080u) | ((v.w << 1) & 0x3C3C3C3Cu);
+    return v;
+}
+template <class SH>
+__device__ __forceinline__ uint4* random_words() { return reinterpret_cast<uint4*>(g_smem + SH::RNDW); }
+
+// All groups of a step (PRE), in two parts.
+template <class SH, int PART>
+__device__ __forceinline__ void draw_step(uint32_t t, int d, uint2 key)
+{
+    constexpr int N = SH::NG * SH::G, H = (N / SH::THREADS + 1) / 2 * SH::THREADS;
+    for (int i = threadIdx.x + (PART ? H : 0); i < (PART ? N : (H < N ? H : N)); i += SH::THREADS)
+        random_words<SH>()[i] = draw_bytes(t, d, i / SH::G, i % SH::G, key);
+}
+
+// The byte that selector sel names (byte_selector) as the low byte, its top
+// bit spread over the next byte, zeros above.
+__device__ __forceinline__ uint32_t spread_byte(uint32_t w, uint32_t sel)
+{
+    uint32_t r;
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(w), "r"(sel));
+    return r;
+}
+__device__ __forceinline__ uint32_t byte_selector(uint32_t q) { return 0x4400u | (8u | q) << 4 | q; }
+
+// The step's colours, in bytes of x offset, drawn by one warp of the CTA;
+// lane 31 returns the words of the step's domain shift.
+template <class SH, int NC>
+__device__ __forceinline__ uint4 draw_schedule(uint32_t t, int d, uint2 key)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const bool shift = lane == 31;
+    const uint4 w = philox(make_uint4(t, shift ? 0u : (uint32_t)d, shift ? ELP_STREAM_SHIFT : (lane | ELP_STREAM_COLOUR), 0u), key);
+    if (lane < SH::NG)
+        reinterpret_cast<uint4*>(g_smem + SH::COLW)[lane] =
+            make_uint4(4 * bounded(w.x, NC), 4 * bounded(w.y, NC), 4 * bounded(w.z, NC), 4 * bounded(w.w, NC));
+    return w;
+}
+
+// The tile at hand, in shared memory: what its load and store need, which
+// would otherwise hold registers through the substeps.
+struct Tile {
+    uint32_t* lat;
+    uint32_t* rec;
+    uint2 key;
+    uint32_t t;         // absolute step
+    int d, L;           // domain, box edge
+    int x0, y0, z0;     // box site of the tile's first word
+};
+static_assert(sizeof(Tile) <= 64, "16 words of shared memory");
+template <class SH>
+__device__ __forceinline__ Tile& tile() { return *reinterpret_cast<Tile*>(g_smem + SH::TILEW); }
+
+// Set up the next tile (one warp): item it of the launch at its step so.
+template <class SH, int TX, int TY, int TZ, int NC>
+__device__ __forceinline__ void next_tile(const BatchLaunch& a, uint2 item, uint32_t step)
+{
+    const BatchJob& J = a.jobs[item.x];
+    const int d = (int)item.y, ntx = J.ntx, nty = J.nty;
+    const uint32_t t = J.step0 + step;
+    const uint2 key = make_uint2(J.seed, J.salt);
+    const uint4 w = draw_schedule<SH, NC>(t, d, key);
+    if ((threadIdx.x & 31) == 31) {
+        Tile& T = tile<SH>();
+        T.lat = J.lat;
+        T.rec = J.rec;
+        T.key = key;
+        T.t = t;
+        T.d = d;
+        T.L = J.L;
+        T.x0 = (int)bounded(w.x, TX) + (d % ntx) * TX;
+        T.y0 = (int)bounded(w.y, TY) + ((d / ntx) % nty) * TY;
+        T.z0 = (int)bounded(w.z, TZ) + (d / ntx / nty) * TZ;
+        g_smem[SH::NSLW] = 0;
+    }
+}
+
+// threadIdx.x as the compiler cannot know it: what is computed from it here
+// is not kept in registers from one tile to the next.
+__device__ __forceinline__ int fresh_tid()
+{
+    int v;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(v));
+    return v;
+}
+
+// This thread's anchors of a substep.  Byte offsets: anchor base + 4 xr; the
+// x offset of colour 0 in the anchor's row (rot); whole box: address of the
+// boundary class's offsets inside the box along x (cls) and the colour
+// offsets at which the anchor's x is 0 or L - 1.
+template <int K>
+struct Anchors {
+    int base[K], rot[K], cls[K], xlo[K], xhi[K], an[K];
+    uint32_t sel[K];   // byte of the counter's words
+    int gq;            // the counter they share
+};
+// Anchor an = g + q G of a substep takes byte q of Philox counter g.  Thread
+// tid owns anchors an = tid + q AT, or with PERM the anchors of the same x
+// group whose row is the tid-th of the 8 x 4 row blocks.
+template <class SH, int TX, int TY, int TZ, bool PER, int NC, int SX, int SXY, int K>
+__device__ __forceinline__ void set_anchors(Anchors<K>& o)
+{
+    const int tid = SH::TAIL && (int)threadIdx.x >= SH::AT ? 0 : (int)threadIdx.x;
+    int tperm = tid;
+    if (SH::PERM) {
+        const int r = tid % SH::R, lane = r & 31, w = r >> 5;
+        const int y = (lane & 7) + 8 * (w % (TY / 8)), z = (lane >> 3) + 4 * (w / (TY / 8));
+        tperm = tid - r + y + TY * z;
+    }
+    o.gq = tperm % SH::G;
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+        const int an = tperm + q * SH::AT;
+        o.an[q] = an;
+        o.sel[q] = byte_selector((uint32_t)(an / SH::G));
+        const int j = an / SH::R, row = an % SH::R;
+        const int y = row % TY, z = row / TY;
+        const int m = (2 * y + 3 * z) % NC;
+        o.rot[q] = 4 * (m ? NC - m : 0);
+        o.base[q] = 4 * (SH::OX + SX * y + SXY * z + NC * j);
+        const int cy = y == 0 ? 0 : (y == TY - 1 ? 2 : 1);
+        const int cz = z == 0 ? 0 : (z == TZ - 1 ? 2 : 1);
+        o.cls[q] = PER ? 4 * SH::OFFW + 64 * (1 + 3 * cy + 9 * cz) : 0;
+        o.xlo[q] = j == 0 ? 0 : -1;
+        o.xhi[q] = j == TX / NC - 1 ? 4 * (NC - 1) : -1;
+    }
+}
+
+// Colour offset of an anchor: (c4 + rot) mod 4 NC.
+template <int NC>
+__device__ __forceinline__ int colour_x(int c4, int rot)
+{
+    int xr4 = c4 + rot;
+    if ((NC & (NC - 1)) == 0) xr4 &= 4 * (NC - 1);
+    else xr4 -= xr4 >= 4 * NC ? 4 * NC : 0;
+    return xr4;
 }
 
 // All substeps of a ring tile whose monomer-0 runs outnumber the slots, with
@@ -217,32 +393,31 @@ __device__ __forceinline__ uint4 group_words(uint4* rnd, int k, uint32_t t, int 
 // in the chain records, halo words ELP_WALL).  Not inlined: it runs rarely,
 // and its registers stay out of the main substep loop.  Same anchors, random
 // words and order as the main loop.  Returns this thread's accepted moves.
-// This thread's anchors, passed by value so that the caller's copies stay in
+// The anchors are passed by value so that the caller's copies stay in
 // registers.
-template <int K>
-struct AnchorSet {
-    int bse[K], rot[K], bsh[K];
-};
-
-template <int K, int NC, int WOFFW, bool PRE, int G>
-__device__ __noinline__ uint32_t general_substeps(const Dom D, const AnchorSet<K> an, const uint32_t* col, uint4* rnd,
-                                                  uint32_t t, int d, int gq, uint2 key)
+template <class SH, int K, int NC, int SX, int SXY>
+__device__ __noinline__ uint32_t general_substeps(const Anchors<K> an, const uint8_t* table)
 {
-    const int* bse = an.bse;
-    const int* rot = an.rot;
-    const int* bsh = an.bsh;
-    const int* woffs = reinterpret_cast<const int*>(g_smem + WOFFW);
+    const int* woffs = reinterpret_cast<const int*>(g_smem + SH::WOFFW);
+    const Tile T = tile<SH>();
+    const int sh4 = 4 * (T.x0 & 3);
+    Dom D;
+    D.S = g_smem; D.tab = table; D.rec = T.rec;
+    D.ox = SH::OX + (T.x0 & 3); D.sx = SX; D.sxy = SXY; D.L = T.L;
+    D.x0 = T.x0; D.y0 = T.y0; D.z0 = T.z0;
+    uint4* rnd = random_words<SH>();
     uint32_t acc = 0;
-    for (int k = 0; k < 2 * NC; k += 4) {
-        const uint4 rw = group_words<K, PRE, G, 2 * NC>(rnd, k, t, d, gq, key);
-        const uint32_t rws[4] = {rw.x, rw.y, rw.z, rw.w};
-        for (int kk = 0; kk < 4; kk++) {
-            const int c4 = (int)col[k + kk];
+    for (int g = 0; g < SH::NG; g++) {
+        const uint4 v = rnd[(SH::PRE ? g * SH::G : 0) + an.gq];
+        for (int kk = 0; kk < 4 && 4 * g + kk < SH::NSUB; kk++) {
+            const int c4 = (int)g_smem[SH::COLW + 4 * g + kk];
+            if (!SH::PRE && kk == 1 && (int)threadIdx.x < SH::G && g + 1 < SH::NG)
+                rnd[threadIdx.x] = draw_bytes(T.t, T.d, g + 1, (int)threadIdx.x, T.key);
             for (int q = 0; q < K; q++) {
-                int xr4 = c4 + rot[q];
-                if ((NC & (NC - 1)) == 0) xr4 &= 4 * (NC - 1);
-                else xr4 -= xr4 >= 4 * NC ? 4 * NC : 0;
-                acc += (uint32_t)op(D, (bse[q] + xr4) >> 2, woffs, (rws[kk] >> bsh[q]) & 0xffu);
+                const int xr4 = colour_x<NC>(c4, an.rot[q]);
+                const uint32_t b = spread_byte(word_of(v, kk), an.sel[q]);
+                if (!SH::TAIL || (int)threadIdx.x < SH::AT)
+                    acc += (uint32_t)op(D, (an.base[q] + sh4 + xr4) >> 2, woffs, ((b >> 7) & 1u) | ((b >> 1) & 0x1Eu));
             }
             __syncthreads();
         }
@@ -250,452 +425,457 @@ __device__ __noinline__ uint32_t general_substeps(const Dom D, const AnchorSet<K
     return acc;
 }
 
-// The K anchors of one thread, one substep.  Returns accepted moves.  Anchor
-// q takes its random byte at bit offset bsh[q] of the Philox word w: bit 0
-// slot (0: the last monomer of P's run, 1: the first monomer of the next
-// run), bits 1-4 table option.  Byte offsets: anchors base4 + 4 xr, colour
-// c4 = 4 c, neighbour offsets at OFFW words; transition table (bytes) at
-// TABW words.  `lin`: the melt holds linear chains (head moves of monomer 0).
-template <int K, bool PER, int NC, int TABW, int OFFW, int HTABW>
-__device__ __forceinline__ int substepK(uint32_t* slot_so, const int (&base4)[K], const int (&rot4)[K],
-                                           const int (&clsyz)[K], const int (&xj4)[K], const int (&bsh)[K],
-                                           const int (&an)[K], int c4, uint32_t w, int L, bool lin, uint32_t t, int d,
-                                           int k, uint2 key)
+// The K anchors of one thread, one substep, random bytes in word w.  Returns
+// accepted moves.  c4 = 4 c, k the substep; LIN: the melt holds linear chains
+// (head moves of monomer 0).
+//
+// The kernel is bound by instruction issue and shared-memory wavefronts, so
+// the move is written for few instructions (49 per warp and substep, 72
+// before; L = 256: 145.8 -> 126 us per step with the tile copy below): one 32-bit entry of the move table carries everything the
+// move's rows decide (target, test, the new words' parts), new words come
+// from additions, and the target and next run are stored ahead of the anchor
+// so that a move back into the anchor's run (target = anchor) needs no case
+// of its own.
+template <class SH, int K, bool PER, int NC, bool LIN>
+__device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, uint32_t w, uint32_t voff, int c4, uint32_t t,
+                                             int d, int k, uint2 key)
 {
-    const uint8_t* tab = reinterpret_cast<const uint8_t*>(g_smem + TABW);
-    const int* offs = reinterpret_cast<const int*>(g_smem + OFFW);
-    int p[K], ob[K];
-    uint32_t wP[K], rb[K];
+    constexpr int TAB4 = 4 * SH::TABW;
+    int p[K], tc[K];
+    uint32_t wP[K], R[K];
 #pragma unroll
     for (int q = 0; q < K; q++) {
-        int xr4 = c4 + rot4[q];
-        if ((NC & (NC - 1)) == 0) xr4 &= 4 * (NC - 1);
-        else xr4 -= xr4 >= 4 * NC ? 4 * NC : 0;
-        p[q] = base4[q] + xr4;
-        int cls = 0;
-        if (PER) {
-            int x4 = xr4 + xj4[q];
-            cls = clsyz[q] + (x4 == 0 ? 0 : (x4 == 4 * (L - 1) ? 2 : 1));
-        }
-        ob[q] = 16 * cls;
+        const int xr4 = colour_x<NC>(c4, an.rot[q]);
+        p[q] = an.base[q] + sh4 + xr4;
         wP[q] = SW(p[q]);
-        rb[q] = (w >> bsh[q]) & 0xffu;
+        if (SH::TAIL && (int)threadIdx.x >= SH::AT) wP[q] = 0;   // an empty site: no move
+        R[q] = spread_byte(w, an.sel[q]);
+        // whole box: the boundary class's offsets (64 bytes each)
+        tc[q] = PER ? an.cls[q] + (xr4 == an.xlo[q] ? -64 : 0) + (xr4 == an.xhi[q] ? 64 : 0) : 0;
     }
     int pB[K];
-    uint32_t wB[K];
+    uint32_t wB[K], V[K];
 #pragma unroll
     for (int q = 0; q < K; q++) {
-        pB[q] = p[q] + offs[ob[q] + (wP[q] & 15)];
-        wB[q] = SW(pB[q]);
+        // {word offset of the step b_out << 16 | row of b_out << 10}: each
+        // lane of a tile's warp holds one code's
+        V[q] = PER ? SW(tc[q] + (int)((wP[q] & 15) << 2)) : __shfl_sync(0xffffffffu, voff, (int)wP[q]);
+        pB[q] = SH::SOFF ? p[q] + ((int)V[q] >> 14) : (int)((uint32_t)(p[q] + (V[q] >> 14)) & 0x3FFFFu);
+        // slot 0 looks at P's own run instead of the next one
+        const uint32_t w1 = SW(pB[q]);
+        wB[q] = (R[q] & 0x8000u) ? w1 : wP[q];
     }
-    uint32_t e[K];
+    uint32_t E[K];
+    bool c2[K];
 #pragma unroll
     for (int q = 0; q < K; q++) {
-        const uint32_t s = rb[q] & 1, bo = wP[q] & 15;
-        const bool c2 = (s ? wB[q] : wP[q]) >= 2u * ELP_CUNIT;
-        const uint32_t src2 = s ? (c2 ? 0u : (wB[q] & 15)) : (c2 ? bo : 0u);
-        e[q] = tab[((s ? bo : 0u) << 8) | (src2 << 4) | ((rb[q] >> 1) & 15)];
+        // row (s ? b_out : 0, src2): src2 is the next run's b_out if that run
+        // holds one monomer (slot 1), P's own if it holds two or more (slot 0)
+        const bool s = (R[q] & 0x8000u) != 0;
+        c2[q] = wB[q] >= 2u * ELP_CUNIT;
+        uint32_t ix = R[q] & (V[q] | 0x3Cu);
+        if (c2[q] != s) ix += (wB[q] & 15) << 6;
+        E[q] = SW(TAB4 + (int)ix);
     }
     int pY[K];
     uint32_t wY[K];
 #pragma unroll
     for (int q = 0; q < K; q++) {
-        pY[q] = p[q] + offs[ob[q] + (e[q] & 15)];
+        if (PER) {
+            const uint32_t V2 = SW(tc[q] + (int)(E[q] >> 26));
+            pY[q] = SH::SOFF ? p[q] + ((int)V2 >> 14) : (int)((uint32_t)(p[q] + (V2 >> 14)) & 0x3FFFFu);
+        } else {
+            pY[q] = p[q] + ((int)E[q] >> 18);
+        }
         wY[q] = SW(pY[q]);
     }
-    int acc = 0;
+    uint32_t acc = 0;
 #pragma unroll
     for (int q = 0; q < K; q++) {
-        const uint32_t d1 = e[q] & 15, d2 = e[q] >> 4, s = rb[q] & 1;
-        const bool join = d2 == 0;  // m joins the front of the next run
-        const bool ok = e[q] && (join ? wY[q] != HWALL : (d1 == 0 || wY[q] == 0));
-        uint32_t nP = wP[q] & ~15u;
-        nP = (s == 0) ? nP - ELP_CUNIT : (d1 ? nP : nP + ELP_CUNIT);
-        nP |= d1 ? d1 : d2;
-        uint32_t nB = (wB[q] >= 2u * ELP_CUNIT) ? wB[q] - ELP_CUNIT : 0u;
-        uint32_t nY = d2 ? (d2 | ELP_CUNIT) : wY[q] + ELP_CUNIT;
-        const uint32_t labs = (wP[q] | (s ? wB[q] : 0u) | (join ? wY[q] : 0u)) & ELP_LBIT;
-        if (ok && labs) follow_label(slot_so, p[q], pB[q], pY[q], wP[q], wB[q], wY[q], s, d1, nP, nB, nY);
+        const bool s = (R[q] & 0x8000u) != 0;
+        const bool ok = E[q] != 0 && (wY[q] & E[q] & (PER ? 0xFu : 0x1Fu)) == 0;
+        const uint32_t nP = ((wP[q] & ~15u) | ((E[q] >> 5) & 15u)) + (E[q] & 0x30000u) - ELP_CUNIT;
+        const uint32_t nB = c2[q] ? wB[q] - ELP_CUNIT : 0u;
+        const uint32_t nY = wY[q] + ELP_CUNIT + ((E[q] >> 9) & 15u);
+        if (ok) SW(pY[q]) = nY;
         if (ok && s) SW(pB[q]) = nB;
-        if (ok && d1) SW(pY[q]) = nY;
         if (ok) SW(p[q]) = nP;
-        wP[q] = ok ? nP : wP[q];
-        acc += ok ? 1 : 0;
+        const bool lab = ok && ((wP[q] | wB[q] | wY[q]) & SH::LMASK);
+        // a branch of the whole warp: predicated, its instructions would be
+        // issued on every substep
+        if (__any_sync(0xffffffffu, lab)) {
+            const bool d1 = PER ? (E[q] >> 28) != 0 : ((int)E[q] >> 18) != 0;
+            if (lab)
+                follow_label<SH>(p[q], pB[q], pY[q], wP[q], wB[q], wY[q], s, d1, (E[q] & (15u << 9)) == 0, nP, nB, nY);
+        }
+        if (LIN && ok) wP[q] = lab ? SW(p[q]) : nP;
+        acc += ok ? 1u : 0u;
     }
     // linear chains: monomer 0 has no predecessor and moves about monomer 1,
     // tried at the anchor holding it after that anchor's regular attempt:
     // with probability 1/2 (bit 0 of its own Philox word) one option of row
     // (0xf, run length > 1 ? 0 : b_out) -- it leaves to the empty site P - u
-    // (its bond to monomer 1 becoming u), or, alone on P, joins the next run
-    if (lin) {
-        const uint8_t* htab = reinterpret_cast<const uint8_t*>(g_smem + HTABW);
+    // (its bond to monomer 1 becoming u), or, alone on P, joins the next run.
+    // Monomer 0 of a linear chain is the first of its run: its offset stays 0.
+    if (LIN) {
+        const uint8_t* htab = reinterpret_cast<const uint8_t*>(g_smem + SH::HTABW);
 #pragma unroll
         for (int q = 0; q < K; q++) {
             const uint32_t w0 = wP[q];
-            if (!(w0 & ELP_LBIT)) continue;
-            const uint4 h = philox(make_uint4(t, (uint32_t)d, (uint32_t)k | ELP_STREAM_HEAD, (uint32_t)an[q]), key);
+            if (!(w0 & SH::LMASK)) continue;
+            const uint4 h = philox(make_uint4(t, (uint32_t)d, (uint32_t)k | ELP_STREAM_HEAD, (uint32_t)an.an[q]), key);
             if (!(h.x & 1)) continue;
             const uint32_t cP = w0 >> ELP_CSHIFT, bo = w0 & 15;
             const uint32_t e = htab[((cP >= 2 ? 0u : bo) << 4) | ((h.x >> 1) & 15)];
             if (!e) continue;
-            const uint32_t d2 = e >> 4, slot = (w0 >> 5) & 0x7FFu;
-            // monomer 0 of a linear chain is the first of its run: offset 0 stays
+            const uint32_t d2 = e >> 4, code = cP >= 2 ? (~d2) & 15u : bo;
+            const uint32_t Vh = SW((PER ? tc[q] : 4 * SH::OFFW) + (int)(code << 2));
+            const int pH = SH::SOFF ? p[q] + ((int)Vh >> 14) : (int)((uint32_t)(p[q] + (Vh >> 14)) & 0x3FFFFu);
+            const uint32_t wH = SW(pH);
             if (cP >= 2) {
-                const int pY = p[q] + offs[ob[q] + ((~d2) & 15u)];
-                if (SW(pY) == 0) {
-                    SW(pY) = d2 | (w0 & LMASK) | ELP_CUNIT;
-                    SW(p[q]) = (w0 & ~LMASK) - ELP_CUNIT;
-                    slot_so[slot] = (slot_so[slot] & 0xFFFFu) | ((uint32_t)(pY >> 2) << 16);
+                if (wH == 0) {
+                    SW(pH) = d2 | (w0 & SH::LMASK) | ELP_CUNIT;
+                    SW(p[q]) = (w0 & ~SH::LMASK) - ELP_CUNIT;
                     acc++;
                 }
-            } else {
-                const int pB = p[q] + offs[ob[q] + bo];
-                const uint32_t wB = SW(pB);
-                if (wB != HWALL) {
-                    SW(pB) = (wB + ELP_CUNIT) | (w0 & LMASK);
-                    SW(p[q]) = 0;
-                    slot_so[slot] = (slot_so[slot] & 0xFFFFu) | ((uint32_t)(pB >> 2) << 16);
-                    acc++;
-                }
+            } else if (wH != HWALL) {
+                SW(pH) = (wH + ELP_CUNIT) | (w0 & SH::LMASK);
+                SW(p[q]) = 0;
+                acc++;
             }
         }
     }
     return acc;
 }
 
-// K anchors per thread: K = 4 keeps four independent moves in flight per
-// thread (instruction-level parallelism); K = 2 or 1 spreads a substep over
-// more warps (latency hiding when a domain has few anchors per SM).  The
-// random stream does not depend on K: anchor a = g + q * G always takes byte
-// q of Philox word (k & 3) of counter {t, d, k / 4, g}.
-template <int TX, int TY, int TZ, bool PER, int NC, int SX, int SXY, int CAP, int K, int THREADS, int MINB, bool LIN>
-__global__ void __launch_bounds__(THREADS, MINB) sweep2_kernel(BatchLaunch a)
+// The substeps of one step of a domain.  Returns this thread's accepted moves.
+template <class SH, int K, bool PER, int NC, bool LIN>
+__device__ __forceinline__ uint32_t substeps(const Anchors<K>& an, int sh4, uint32_t voff)
 {
-    using SH = Shape<TX, TY, TZ, PER, NC, SX, SXY, CAP, K, MINB>;
-    static_assert(K == 1 || K == 2 || K == 4, "anchors per thread");
-    static_assert(SH::A % 4 == 0 && SH::AT == THREADS && THREADS % 32 == 0, "every thread owns K anchors");
-    static_assert(CAP <= 2048, "slot numbers are 11 bits");
-    static_assert((2 * NC) % 4 == 0, "substeps come in groups of four");
-    static_assert(THREADS % TX == 0, "tile columns are split evenly over the threads");
-    constexpr int TABW = SH::TABW, OFFW = SH::OFFW, HTABW = SH::HTABW;
+    uint4* rnd = random_words<SH>();
+    uint32_t acc = 0;
+    // what draws need in here (linear chains; groups drawn one at a time)
+    uint32_t t = 0;
+    int d = 0;
+    uint2 key = make_uint2(0, 0);
+    if (LIN || !SH::PRE) {
+        t = tile<SH>().t;
+        d = tile<SH>().d;
+        key = tile<SH>().key;
+    }
+#pragma unroll 1
+    for (int g = 0; g < SH::NG; g++) {
+        const uint4 c4 = reinterpret_cast<const uint4*>(g_smem + SH::COLW)[g];
+        const uint4 v = rnd[(SH::PRE ? g * SH::G : 0) + an.gq];
+        acc += substepK<SH, K, PER, NC, LIN>(an, sh4, v.x, voff, (int)c4.x, t, d, 4 * g, key);
+        __syncthreads();
+        // the next group's bytes: every thread has read this group's
+        if (!SH::PRE && (int)threadIdx.x < SH::G && g + 1 < SH::NG)
+            rnd[threadIdx.x] = draw_bytes(t, d, g + 1, (int)threadIdx.x, key);
+        acc += substepK<SH, K, PER, NC, LIN>(an, sh4, v.y, voff, (int)c4.y, t, d, 4 * g + 1, key);
+        __syncthreads();
+        if (SH::NSUB % 4 && 4 * g + 2 >= SH::NSUB) break;
+        acc += substepK<SH, K, PER, NC, LIN>(an, sh4, v.z, voff, (int)c4.z, t, d, 4 * g + 2, key);
+        __syncthreads();
+        acc += substepK<SH, K, PER, NC, LIN>(an, sh4, v.w, voff, (int)c4.w, t, d, 4 * g + 3, key);
+        __syncthreads();
+    }
+    return acc;
+}
+
+// Add a thread's accepted moves to the melt's counter, one atomic per warp.
+__device__ __forceinline__ void count_accepted(unsigned long long* acc, unsigned long long v)
+{
+    if (!acc) return;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(acc, v);
+}
+
+// Tables of a launch into shared memory: moves and neighbour offsets
+// (elp_move_table builds them in this order) and rows (0xf, x) of the
+// transition table (moves of a linear chain's monomer 0).
+template <class SH, bool PER>
+__device__ __forceinline__ void load_tables(const BatchLaunch& a)
+{
+    for (int i = threadIdx.x; i < (ELP_MOVE_ENTRIES + SH::NOFF + (PER ? 0 : 16)) / 4; i += SH::THREADS)
+        cp_async16(g_smem + SH::TABW + 4 * i, a.moves + 4 * i);
+    for (int i = threadIdx.x; i < 64; i += SH::THREADS) g_smem[SH::HTABW + i] = a.table[960 + i];
+}
+
+// Whole boxes: each CTA holds one melt for all steps of the launch.
+//
+// K anchors per thread: K = 2 where a domain has more than 1024 anchors per
+// substep, else 1 (more warps hide latency better than more moves in flight
+// per thread).  The random stream does not depend on K.
+template <int TX, int NC, int SX, int SXY, int CAP, int K, bool LIN>
+__global__ void __launch_bounds__(((TX * TX * (TX / NC) / K) + 31) / 32 * 32, 1) sweep_box(BatchLaunch a)
+{
+    using SH = Shape<TX, TX, TX, true, NC, SX, SXY, CAP, K, 1>;
+    constexpr int SITES = TX * TX * TX;
     uint32_t* S = g_smem;
-    uint8_t* tab = reinterpret_cast<uint8_t*>(g_smem + TABW);
-    int* offs = reinterpret_cast<int*>(g_smem + OFFW);
-    uint32_t* col = g_smem + SH::COLW;
-    uint32_t* shf = g_smem + SH::SHFW;
-    uint32_t* slot_chain = g_smem + SH::SCHW;
-    uint32_t* slot_so = g_smem + SH::SSOW;
-    uint32_t* nslots = g_smem + SH::NSLW;
-    uint4* rnd = reinterpret_cast<uint4*>(g_smem + SH::RNDW);
     const int tid = threadIdx.x;
-    const int cx = tid % TX;  // the tile column this thread loads, scans and stores
-    const int LP = TX;  // box edge of whole-box (periodic) domains
-
-    // table words: entries 4i .. 4i+3 of row i / 4 = (src1 << 4) | src2.
-    // Cleared: rows with a source that is no bond (3, 12: halo words) and
-    // rows with src1 = 0xf (slot 1 at the last run of a linear chain, which
-    // has no next run); rows (0xf, x) are kept apart for monomer-0 moves.
-    for (int i = tid; i < 1024; i += THREADS) {
-        const int s1 = i >> 6, s2 = (i >> 2) & 15;
-        const bool nobond = s1 == 3 || s1 == 12 || s1 == 15 || s2 == 3 || s2 == 12;
-        reinterpret_cast<uint32_t*>(tab)[i] = nobond ? 0u : a.table[i];
-    }
-    for (int i = tid; i < 64; i += THREADS) g_smem[HTABW + i] = a.table[960 + i];
-    for (int i = tid; i < SH::NOFF; i += THREADS) {
-        // whole box: class (cx, cy, cz) of the anchor on each axis (0 first
-        // plane, 2 last, 1 inside) wraps the offsets; tiles: one class
-        int cls = PER ? (i >> 4) : 13, b = i & 15;
-        int dt = elp_bt(b), du = elp_bu(b), dv = elp_bv(b);
-        if (PER) {
-            int cx = cls % 3, cy = (cls / 3) % 3, cz = cls / 9;
-            if (cx == 0 && dt < 0) dt = LP - 1;
-            if (cx == 2 && dt > 0) dt = -(LP - 1);
-            if (cy == 0 && du < 0) du = LP - 1;
-            if (cy == 2 && du > 0) du = -(LP - 1);
-            if (cz == 0 && dv < 0) dv = LP - 1;
-            if (cz == 2 && dv > 0) dv = -(LP - 1);
-        }
-        offs[i] = 4 * (dt + SX * du + SXY * dv);   // bytes
-        if (!PER) reinterpret_cast<int*>(g_smem + SH::WOFFW)[i] = dt + SX * du + SXY * dv;
-    }
-    if (!PER)
-        for (int i = tid; i < SH::WORDS; i += THREADS) S[i] = HWALL;
-
-    // Anchor an = g + q G of a substep takes byte q of Philox word g.  Thread
-    // tid owns anchors an = tid + q AT, or with PERM the anchors of the same
-    // x group whose row is the tid-th of the 8 x 4 row blocks.
-    int base[K], rot[K], clsyz[K], xj[K], bsh[K], anq[K];
-    int tperm = tid;
-    if (SH::PERM) {
-        const int r = tid % SH::R, lane = r & 31, w = r >> 5;
-        const int y = (lane & 7) + 8 * (w % (TY / 8)), z = (lane >> 3) + 4 * (w / (TY / 8));
-        tperm = tid - r + y + TY * z;
-    }
-    const int gq = tperm % SH::G;   // Philox counter word 3 of this thread's anchors
-#pragma unroll
-    for (int q = 0; q < K; q++) {
-        int an = tperm + q * SH::AT;
-        anq[q] = an;
-        bsh[q] = 8 * (an / SH::G);
-        int j = an / SH::R, row = an % SH::R;
-        int y = row % TY, z = row / TY;
-        int m = (2 * y + 3 * z) % NC;
-        rot[q] = 4 * (m ? NC - m : 0);                       // bytes
-        base[q] = 4 * (SH::OX + SX * y + SXY * z + NC * j);  // bytes
-        int cy = y == 0 ? 0 : (y == LP - 1 ? 2 : 1);
-        int cz = z == 0 ? 0 : (z == LP - 1 ? 2 : 1);
-        clsyz[q] = PER ? (3 * cy + 9 * cz) : 13;
-        xj[q] = 4 * NC * j;
-    }
+    load_tables<SH, true>(a);
+    Anchors<K> an;
+    set_anchors<SH, TX, TX, TX, true, NC, SX, SXY, K>(an);
     const uint32_t step_dev = a.step_dev ? *a.step_dev : 0u;
-    const uint32_t polls = a.wait_polls ? a.wait_polls : WAIT_POLLS;
-    // Whole-box domains run their steps back to back on chip; tiled domains
-    // move their tiles every step, so a launch of several steps takes its
-    // steps one after another over all tiles, with a grid barrier between
-    // steps (the launch is cooperative: all CTAs are resident).
-    const int outer = PER ? 1 : a.nsteps, inner = PER ? a.nsteps : 1;
-
-    for (int so = 0; so < outer; so++) {
-    if (so > 0) {
-        // a test may keep one CTA from arriving at the first barrier
-        const bool arrive = !(so == 1 && (int)blockIdx.x + 1 == a.hold_cta1);
-        if (!grid_barrier(a.grid_bar, gridDim.x * (uint32_t)so, polls, arrive)) {
-            if (tid == 0) atomicOr(a.error, 4u);
-            break;
-        }
-    }
     for (int it = blockIdx.x; it < a.nitems; it += gridDim.x) {
-        const uint2 item = a.items[it];
-        const BatchJob& J = a.jobs[item.x];
-        const int d = (int)item.y;
-        const int L = PER ? LP : J.L;
+        const BatchJob& J = a.jobs[a.items[it].x];
         uint32_t* lat = J.lat;
         uint32_t* rec = J.rec;
-        const int nchains = J.nchains;
         const uint2 key = make_uint2(J.seed, J.salt);
-        const bool lin = LIN && J.linear != 0;   // the ring instantiation has no monomer-0 moves
-        const int ntx = J.ntx, nty = J.nty;
-        Dom D;
-        D.S = S; D.tab = tab; D.rec = rec;
-        D.ox = SH::OX; D.sx = SX; D.sxy = SXY; D.L = L;
-        D.x0 = 0; D.y0 = 0; D.z0 = 0;
-        uint32_t accepted = 0;
-        bool overflow = false, spill = false;
-        int bse[K];   // anchor base byte offsets of this tile (plus its offset sh in the spans)
-#pragma unroll
-        for (int q = 0; q < K; q++) bse[q] = base[q];
+        const uint32_t t0 = J.step0 + a.step_base + step_dev;
+        __syncthreads();   // the previous melt's words and slots have been read
+        if (tid == 0) g_smem[SH::NSLW] = 0;
+        __syncthreads();
+        for (int i = tid; i < SITES; i += SH::THREADS) {
+            const int idx = i % TX + SX * (i / TX % TX) + SXY * (i / (TX * TX));
+            const uint32_t wv = __ldcg(lat + i);
+            S[idx] = wv;
+            if (wv & ELP_LBIT) claim_slot<SH>(wv, idx);
+        }
+        cp_async_wait_all();
+        __syncthreads();
+        const uint32_t ns = g_smem[SH::NSLW];
+        if (ns > (uint32_t)SH::SLOTS) {
+            // more monomer-0 runs than slots: leave the box untouched, report
+            if (tid == 0) atomicOr(a.error, 1u);
+            continue;
+        }
+        fill_slots<SH>(rec, ns);
+        unsigned long long accepted = 0;
+        for (int st = 0; st < a.nsteps; st++) {
+            const uint32_t t = t0 + (uint32_t)st;
+            if (tid < SH::G) random_words<SH>()[tid] = draw_bytes(t, 0, 0, tid, key);
+            if (tid >= SH::THREADS - 32) draw_schedule<SH, NC>(t, 0, key);
+            if (tid == 0) {
+                tile<SH>().t = t;
+                tile<SH>().d = 0;
+                tile<SH>().key = key;
+            }
+            __syncthreads();
+            accepted += substeps<SH, K, true, NC, LIN>(an, 0, 0u);
+        }
+        for (int i = tid; i < SITES; i += SH::THREADS) {
+            uint32_t wv = S[i % TX + SX * (i / TX % TX) + SXY * (i / (TX * TX))];
+            if (wv & SH::LMASK) wv = leave_slot<SH>(wv, (uint32_t)i, rec);
+            lat[i] = wv;
+        }
+        count_accepted(J.acc, accepted);
+    }
+}
 
-        for (int st = 0; st < inner && !overflow; st++) {
-            const uint32_t t = J.step0 + a.step_base + step_dev + (uint32_t)(so + st);
-            if (!PER && tid < 32) {
-                // one warp draws the step's domain shift for the whole CTA
-                const uint4 sh = philox(make_uint4(t, 0, ELP_STREAM_SHIFT, 0), key);
-                if (tid == 0) {
-                    shf[0] = bounded(sh.x, TX);
-                    shf[1] = bounded(sh.y, TY);
-                    shf[2] = bounded(sh.z, TZ);
-                }
+// Tiles: each CTA takes tile after tile of a step; a launch of several steps
+// is cooperative, with a grid barrier between steps.
+//
+// At L = 128 (one tile per CTA and step) what surrounds the substeps took 10.7
+// of a step's 23.2 us, mostly address arithmetic (1180 instructions per warp,
+// now 790) and latencies in a row.  So a thread's quads differ by whole planes
+// only, labelled words are found in registers on the way in and out, the
+// step's random bytes are drawn while the quads are on their way and between
+// arriving at the grid barrier and waiting for it, and what a tile's load and
+// store need sits in shared memory in between (held in registers it made the
+// substep loop recompute its own).  19.4 us per step now, 23.4 before.
+template <int TX, int TY, int TZ, int NC, int SX, int SXY, int CAP, int K, int MINB, bool LIN>
+__global__ void __launch_bounds__(((TY * TZ * (TX / NC) / K) + 31) / 32 * 32, MINB) sweep_tiles(BatchLaunch a)
+{
+    using SH = Shape<TX, TY, TZ, false, NC, SX, SXY, CAP, K, MINB>;
+    uint32_t* S = g_smem;
+    const int tid = threadIdx.x;
+    load_tables<SH, false>(a);
+    for (int i = tid; i < SH::WORDS / 4; i += SH::THREADS)
+        reinterpret_cast<uint4*>(S)[i] = make_uint4(HWALL, HWALL, HWALL, HWALL);
+    cp_async_wait_all();
+    __syncthreads();
+    const uint32_t voff = g_smem[SH::OFFW + (tid & 15)];   // step of code lane & 15
+    Anchors<K> an;
+    set_anchors<SH, TX, TY, TZ, false, NC, SX, SXY, K>(an);
+    const bool scheduler = tid >= SH::THREADS - 32;   // the warp that sets up the next tile
+    const uint32_t step0 = a.step_base + (a.step_dev ? *a.step_dev : 0u);
+
+    uint2 item = a.items[blockIdx.x];
+    unsigned long long accepted = 0;
+    bool drawn = false;   // the first part of the tile's random bytes is on chip already
+    if (scheduler) next_tile<SH, TX, TY, TZ, NC>(a, item, step0);
+    __syncthreads();
+    for (int so = 0, it = blockIdx.x;;) {
+        // ---- load: quads of four words; a quad never straddles x = L (L and
+        // xa are multiples of 4)
+        {
+            const Tile T = tile<SH>();
+            const int ft = fresh_tid(), L = T.L;
+            const bool mover = !SH::TAIL || ft < SH::AT, ender = SH::R == SH::THREADS || ft < SH::R;
+            const uint32_t LL = (uint32_t)(L * L);
+            const int xa = T.x0 & ~3, sh = T.x0 & 3;
+            const int mc = ft % SH::CB, my = ft / SH::CB % TY, mz = ft / SH::CB / TY;
+            const int ey = ft % TY, ez = ft / TY;   // the row whose end quad it moves
+            uint4 ve = make_uint4(HWALL, HWALL, HWALL, HWALL);
+            if (ender && sh) {
+                int x = xa + TX; x -= x >= L ? L : 0;
+                int y = T.y0 + ey; y -= y >= L ? L : 0;
+                int z = T.z0 + ez; z -= z >= L ? L : 0;
+                ve = __ldcg(reinterpret_cast<const uint4*>(T.lat + ((uint32_t)(x + L * y) + LL * (uint32_t)z)));
             }
-            if (st == 0) {
-                __syncthreads();  // the previous item's stores have read shared memory; the shift is written
-                if (!PER) {
-                    D.x0 = (int)shf[0] + (d % ntx) * TX;
-                    D.y0 = (int)shf[1] + ((d / ntx) % nty) * TY;
-                    D.z0 = (int)shf[2] + (d / ntx / nty) * TZ;
-                }
-                if (tid == 0) *nslots = 0;
-                const bool few = nchains <= THREADS;  // few rings: find monomer 0 through the records
-                if (PER) {
-                    // each thread owns one x column of the box: rows r = y + TY z
-                    for (int r = tid / TX; r < SH::R; r += THREADS / TX) {
-                        const int y = r % TY, z = r / TY;
-                        cp_async4(S + cx + SX * y + SXY * z, lat + (uint32_t)(cx + L * (y + L * z)));
-                    }
-                    cp_async_wait_all();
-                    __syncthreads();
-                    if (!few) {
-                        for (int r = tid / TX; r < SH::R; r += THREADS / TX) {
-                            const int idx = cx + SX * (r % TY) + SXY * (r / TY);
-                            const uint32_t wv = S[idx];
-                            if (wv & ELP_LBIT) S[idx] = take_slot<CAP>(wv, idx, rec, nslots, slot_chain, slot_so);
-                        }
-                    }
-                } else {
-                    // rows r = y + TY z: the 16-byte aligned span [xa, xa + TX + 4)
-                    // of the box row in 16-byte granules (a granule never
-                    // straddles x = L: L and xa are multiples of 4)
-                    const int xa = D.x0 & ~3, sh = D.x0 & 3;
-                    D.ox = SH::OX + sh;
+            constexpr int NB = SH::NP <= 6 ? SH::NP : 4;   // quads in flight per thread
+            static_assert(SH::NP % NB == 0, "passes per batch");
+            int x = xa + 4 * mc; x -= x >= L ? L : 0;
+            int y = T.y0 + my; y -= y >= L ? L : 0;
+            int z = T.z0 + mz; z -= z >= L ? L : 0;
+            const uint32_t* src = T.lat + (uint32_t)(x + L * y);
+            const int at0 = SH::OX + SX * my + SXY * mz + 4 * mc;
 #pragma unroll
-                    for (int q = 0; q < K; q++) bse[q] = base[q] + 4 * sh;
-                    constexpr int CPR = SH::SPAN / 4;
-                    for (int i = tid; i < SH::R * CPR; i += THREADS) {
-                        const int r = i / CPR, c = i - r * CPR;
-                        const int y = r % TY, z = r / TY;
-                        int gy = D.y0 + y; gy -= gy >= L ? L : 0;
-                        int gz = D.z0 + z; gz -= gz >= L ? L : 0;
-                        int gx = xa + 4 * c; gx -= gx >= L ? L : 0;
-                        cp_async16(S + SH::OX + SX * y + SXY * z + 4 * c, lat + (uint32_t)(gx + L * (gy + L * gz)));
-                    }
-                    // the step's Philox words while the rows are in flight
-                    // (the same counters as the two-buffer schedule draws)
-                    if (SH::PRE)
-                        for (int i = tid; i < SH::NG * SH::G; i += THREADS)
-                            rnd[i] = philox(make_uint4(t, (uint32_t)d, (uint32_t)(i / SH::G), (uint32_t)(i % SH::G)), key);
-                    cp_async_wait_all();
-                    __syncthreads();
-                    // span words outside the tile become halo words; with many
-                    // rings, monomer 0's runs are found in the same pass
-                    for (int i = tid; i < SH::R * CPR; i += THREADS) {
-                        const int r = i / CPR, c = i - r * CPR;
-                        const int at = SH::OX + SX * (r % TY) + SXY * (r / TY) + 4 * c;
-                        const int p0 = 4 * c - sh;  // tile column of the chunk's first word
-                        uint4 v = *reinterpret_cast<const uint4*>(S + at);
-                        const bool edge = p0 < 0 || p0 + 4 > TX;
-                        if (edge) {
-                            v.x = (unsigned)(p0 + 0) < (unsigned)TX ? v.x : HWALL;
-                            v.y = (unsigned)(p0 + 1) < (unsigned)TX ? v.y : HWALL;
-                            v.z = (unsigned)(p0 + 2) < (unsigned)TX ? v.z : HWALL;
-                            v.w = (unsigned)(p0 + 3) < (unsigned)TX ? v.w : HWALL;
-                        }
-                        if (!few && ((v.x | v.y | v.z | v.w) & ELP_LBIT)) {
-                            if (v.x & ELP_LBIT) v.x = take_slot<CAP>(v.x, at + 0, rec, nslots, slot_chain, slot_so);
-                            if (v.y & ELP_LBIT) v.y = take_slot<CAP>(v.y, at + 1, rec, nslots, slot_chain, slot_so);
-                            if (v.z & ELP_LBIT) v.z = take_slot<CAP>(v.z, at + 2, rec, nslots, slot_chain, slot_so);
-                            if (v.w & ELP_LBIT) v.w = take_slot<CAP>(v.w, at + 3, rec, nslots, slot_chain, slot_so);
-                            *reinterpret_cast<uint4*>(S + at) = v;
-                        } else if (edge) {
-                            *reinterpret_cast<uint4*>(S + at) = v;
-                        }
-                    }
-                    if (few) __syncthreads();
-                }
-                if (few) {
-                    for (int ch = tid; ch < nchains; ch += THREADS) {
-                        const uint4 r = __ldcg(reinterpret_cast<const uint4*>(rec + ELP_REC_WORDS * (size_t)ch));
-                        const int gx = (int)(r.x % (uint32_t)L), gy = (int)((r.x / (uint32_t)L) % (uint32_t)L),
-                                  gz = (int)(r.x / ((uint32_t)L * L));
-                        int x = gx - D.x0; x += x < 0 ? L : 0;
-                        int y = gy - D.y0; y += y < 0 ? L : 0;
-                        int z = gz - D.z0; z += z < 0 ? L : 0;
-                        if (x < TX && y < TY && z < TZ) {
-                            const uint32_t slot = atomicAdd(nslots, 1u);
-                            if (slot < (uint32_t)CAP) {
-                                const int idx = D.ox + x + SX * y + SXY * z;
-                                slot_chain[slot] = (uint32_t)ch;
-                                slot_so[slot] = r.z | ((uint32_t)idx << 16);
-                                S[idx] = (S[idx] & 15) | ELP_LBIT | (slot << 5) | (r.y << ELP_CSHIFT);
-                            }
-                        }
-                    }
-                }
-            }
-            if (K < 4 && !SH::PRE && tid < SH::G) rnd[tid] = philox(make_uint4(t, (uint32_t)d, 0u, (uint32_t)tid), key);
-            if (tid < (2 * NC + 3) / 4) {
-                const uint4 cw = philox(make_uint4(t, (uint32_t)d, (uint32_t)tid | ELP_STREAM_COLOUR, 0), key);
-                col[4 * tid + 0] = 4 * bounded(cw.x, NC);   // colours in bytes of x offset
-                col[4 * tid + 1] = 4 * bounded(cw.y, NC);
-                col[4 * tid + 2] = 4 * bounded(cw.z, NC);
-                col[4 * tid + 3] = 4 * bounded(cw.w, NC);
-            }
-            __syncthreads();
-            if (*nslots > (uint32_t)CAP) {
-                if (PER || lin) {
-                    // more monomer-0 runs than slots where the general move
-                    // does not apply: leave this domain untouched, report
-                    if (tid == 0) atomicOr(a.error, 1u);
-                    overflow = true;
-                    break;
-                }
-                // a crowded ring tile: words back to their global form (the
-                // records still hold the runs' lengths and offsets), halo
-                // words to the general move's wall
-                spill = true;
-                for (int sl = tid; sl < CAP; sl += THREADS) {
-                    const int idx = (int)(slot_so[sl] >> 16);
-                    S[idx] = (S[idx] & 15) | ELP_LBIT | (slot_chain[sl] << 5);
-                }
-                for (int i = tid; i < SH::WORDS; i += THREADS)
-                    if (S[i] == HWALL) S[i] = ELP_WALL;
-                __syncthreads();
-            }
-            if (!PER && spill) {
-                AnchorSet<K> as;
+            for (int i0 = 0; i0 < SH::NP; i0 += NB) {
+                uint4 v[NB];
 #pragma unroll
-                for (int q = 0; q < K; q++) {
-                    as.bse[q] = bse[q];
-                    as.rot[q] = rot[q];
-                    as.bsh[q] = bsh[q];
+                for (int i = 0; i < NB; i++) {
+                    if (mover) v[i] = __ldcg(reinterpret_cast<const uint4*>(src + LL * (uint32_t)z));
+                    z += SH::ZS; z -= z >= L ? L : 0;
                 }
-                accepted += general_substeps<K, NC, SH::WOFFW, SH::PRE, SH::G>(D, as, col, rnd, t, d, gq, key);
-                continue;
-            }
-#pragma unroll 1
-            for (int k = 0; k < 2 * NC; k += 4) {
-                const uint4 rw = group_words<K, SH::PRE, SH::G, 2 * NC>(rnd, k, t, d, gq, key);
-                const uint32_t rws[4] = {rw.x, rw.y, rw.z, rw.w};
+                if (SH::PRE && i0 == 0) {   // the step's random bytes while the quads are on their way
+                    if (!drawn) draw_step<SH, 0>(T.t, T.d, T.key);
+                    draw_step<SH, 1>(T.t, T.d, T.key);
+                }
 #pragma unroll
-                for (int kk = 0; kk < 4; kk++) {
-                    accepted += (uint32_t)substepK<K, PER, NC, TABW, OFFW, HTABW>(
-                        slot_so, bse, rot, clsyz, xj, bsh, anq, (int)col[k + kk], rws[kk], LP, lin, t, d, k + kk, key);
-                    __syncthreads();
+                for (int i = 0; i < NB; i++) {
+                    if (mc == 0) {   // words ahead of the tile
+                        if (sh > 0) v[i].x = HWALL;
+                        if (sh > 1) v[i].y = HWALL;
+                        if (sh > 2) v[i].z = HWALL;
+                    }
+                    if (mover) {
+                        const int at = at0 + (i0 + i) * SXY * SH::ZS;
+                        *reinterpret_cast<uint4*>(S + at) = v[i];
+                        if ((v[i].x | v[i].y | v[i].z | v[i].w) & ELP_LBIT) {
+                            if ((v[i].x & ELP_LBIT) && v[i].x != HWALL) claim_slot<SH>(v[i].x, at);
+                            if ((v[i].y & ELP_LBIT) && v[i].y != HWALL) claim_slot<SH>(v[i].y, at + 1);
+                            if ((v[i].z & ELP_LBIT) && v[i].z != HWALL) claim_slot<SH>(v[i].z, at + 2);
+                            if (v[i].w & ELP_LBIT) claim_slot<SH>(v[i].w, at + 3);
+                        }
+                    }
                 }
             }
+            if (ender) {   // words 0 .. sh-1 of the end quad are the tile's
+                const int at = SH::OX + SX * ey + SXY * ez + TX;
+                if (sh < 1) ve.x = HWALL; else if (ve.x & ELP_LBIT) claim_slot<SH>(ve.x, at);
+                if (sh < 2) ve.y = HWALL; else if (ve.y & ELP_LBIT) claim_slot<SH>(ve.y, at + 1);
+                if (sh < 3) ve.z = HWALL; else if (ve.z & ELP_LBIT) claim_slot<SH>(ve.z, at + 2);
+                ve.w = HWALL;
+                *reinterpret_cast<uint4*>(S + at) = ve;
+            }
+            if (!SH::PRE && tid < SH::G) random_words<SH>()[tid] = draw_bytes(T.t, T.d, 0, tid, T.key);
         }
-        if (spill) {
-            // the halo goes back to the form the slot-table path expects
-            for (int i = tid; i < SH::WORDS; i += THREADS)
+        __syncthreads();
+
+        // ---- monomer-0 runs, substeps
+        const uint32_t ns = g_smem[SH::NSLW];
+        const bool crowded = ns > (uint32_t)SH::SLOTS;
+        if (!crowded) {
+            fill_slots<SH>(tile<SH>().rec, ns);
+            __syncthreads();
+            accepted += substeps<SH, K, false, NC, LIN>(an, 4 * (tile<SH>().x0 & 3), voff);
+        } else if (!LIN) {
+            // a crowded ring tile: its words are still in their global form
+            // and the records hold the runs' lengths and offsets; halo words
+            // become the general move's walls
+            for (int i = tid; i < SH::WORDS; i += SH::THREADS)
+                if (S[i] == HWALL) S[i] = ELP_WALL;
+            __syncthreads();
+            accepted += general_substeps<SH, K, NC, SX, SXY>(an, reinterpret_cast<const uint8_t*>(a.table));
+            for (int i = tid; i < SH::WORDS; i += SH::THREADS)
                 if (S[i] == ELP_WALL) S[i] = HWALL;
-        }
-        if (!overflow) {
-            const uint32_t ns = spill ? 0u : *nslots;   // a spilled tile's records are already written
-            for (uint32_t sl = tid; sl < ns; sl += THREADS) {
-                const uint32_t so16 = slot_so[sl];
-                const int idx = (int)(so16 >> 16);
-                const uint32_t wv = S[idx];
-                const uint32_t chain = slot_chain[sl];
-                *reinterpret_cast<uint4*>(rec + ELP_REC_WORDS * (size_t)chain) =
-                    make_uint4(global_site(D, idx), wv >> ELP_CSHIFT, so16 & 0xFFFFu, 0u);
-                S[idx] = (wv & 15) | ELP_LBIT | (chain << 5);
-            }
             __syncthreads();
-            if (PER) {
-                for (int r = tid / TX; r < SH::R; r += THREADS / TX) {
-                    const int y = r % TY, z = r / TY;
-                    lat[(uint32_t)(cx + L * (y + L * z))] = S[cx + SX * y + SXY * z];
-                }
-            } else {
-                // 16-byte stores of the span's chunks inside the tile, single
-                // words at its ragged ends (a chunk never straddles x = L)
-                const int xa = D.x0 & ~3, sh = D.x0 & 3;
-                constexpr int CPR = SH::SPAN / 4;
-                for (int i = tid; i < SH::R * CPR; i += THREADS) {
-                    const int r = i / CPR, c = i - r * CPR;
-                    const int y = r % TY, z = r / TY;
-                    int gy = D.y0 + y; gy -= gy >= L ? L : 0;
-                    int gz = D.z0 + z; gz -= gz >= L ? L : 0;
-                    int gx = xa + 4 * c; gx -= gx >= L ? L : 0;
-                    uint32_t* g = lat + (uint32_t)(gx + L * (gy + L * gz));
-                    const uint32_t* cp = S + SH::OX + SX * y + SXY * z + 4 * c;
-                    const int p0 = 4 * c - sh;
-                    if (p0 >= 0 && p0 + 4 <= TX) {
-                        *reinterpret_cast<uint4*>(g) = *reinterpret_cast<const uint4*>(cp);
-                    } else {
+        } else if (tid == 0) {
+            // linear chains: the general move does not apply; leave the tile
+            // untouched, report
+            atomicOr(a.error, 1u);
+        }
+
+        // ---- store: quads inside the tile, single words at its ragged ends
+        if (!crowded || !LIN) {
+            const Tile T = tile<SH>();
+            const int ft = fresh_tid(), L = T.L;
+            const bool mover = !SH::TAIL || ft < SH::AT, ender = SH::R == SH::THREADS || ft < SH::R;
+            const uint32_t LL = (uint32_t)(L * L), lmask = crowded ? 0u : SH::LMASK;
+            const int xa = T.x0 & ~3, sh = T.x0 & 3;
+            const int mc = ft % SH::CB, my = ft / SH::CB % TY, mz = ft / SH::CB / TY;
+            int x = xa + 4 * mc; x -= x >= L ? L : 0;
+            int y = T.y0 + my; y -= y >= L ? L : 0;
+            int z = T.z0 + mz; z -= z >= L ? L : 0;
+            const uint32_t xy = (uint32_t)(x + L * y);
+            const int at0 = SH::OX + SX * my + SXY * mz + 4 * mc;
 #pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            if ((unsigned)(p0 + k) < (unsigned)TX) g[k] = cp[k];
-                    }
+            for (int i = 0; i < SH::NP; i++) {
+                const uint32_t site = xy + LL * (uint32_t)z;
+                z += SH::ZS; z -= z >= L ? L : 0;
+                if (!mover) continue;
+                uint4 v = *reinterpret_cast<const uint4*>(S + at0 + i * SXY * SH::ZS);
+                if ((v.x | v.y | v.z | v.w) & lmask) {
+                    if (v.x & lmask) v.x = leave_slot<SH>(v.x, site, T.rec);
+                    if (v.y & lmask) v.y = leave_slot<SH>(v.y, site + 1, T.rec);
+                    if (v.z & lmask) v.z = leave_slot<SH>(v.z, site + 2, T.rec);
+                    if (v.w & lmask) v.w = leave_slot<SH>(v.w, site + 3, T.rec);
+                }
+                if (mc != 0 || sh == 0) {
+                    *reinterpret_cast<uint4*>(T.lat + site) = v;
+                } else {
+                    if (sh < 2) T.lat[site + 1] = v.y;
+                    if (sh < 3) T.lat[site + 2] = v.z;
+                    T.lat[site + 3] = v.w;
+                }
+            }
+            if (ender && sh) {
+                const int ey = ft % TY, ez = ft / TY;
+                int x = xa + TX; x -= x >= L ? L : 0;
+                int y = T.y0 + ey; y -= y >= L ? L : 0;
+                int z = T.z0 + ez; z -= z >= L ? L : 0;
+                const uint32_t es = (uint32_t)(x + L * y) + LL * (uint32_t)z;
+                uint4 v = *reinterpret_cast<const uint4*>(S + SH::OX + SX * ey + SXY * ez + TX);
+                if (v.x & lmask) v.x = leave_slot<SH>(v.x, es, T.rec);
+                T.lat[es] = v.x;
+                if (sh > 1) {
+                    if (v.y & lmask) v.y = leave_slot<SH>(v.y, es + 1, T.rec);
+                    T.lat[es + 1] = v.y;
+                }
+                if (sh > 2) {
+                    if (v.z & lmask) v.z = leave_slot<SH>(v.z, es + 2, T.rec);
+                    T.lat[es + 2] = v.z;
                 }
             }
         }
-        if (J.acc) {
-            unsigned long long v = (unsigned long long)accepted;
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if ((tid & 31) == 0 && v) atomicAdd(J.acc, v);
+
+        // ---- the next tile
+        it += gridDim.x;
+        const bool over = it >= a.nitems;   // the step's tiles are done
+        if (over) {
+            it = blockIdx.x;
+            so++;
+        }
+        const bool last = so >= a.nsteps;
+        const uint32_t job = item.x;
+        if (!last) item = a.items[it];
+        if (last || item.x != job) {
+            count_accepted(a.jobs[job].acc, accepted);
+            accepted = 0;
+        }
+        if (last) break;
+        __syncthreads();   // the tile's words and description have been read
+        if (scheduler) next_tile<SH, TX, TY, TZ, NC>(a, item, step0 + (uint32_t)so);
+        // a test may keep one CTA from arriving at the first barrier
+        if (over && tid == 0 && !(so == 1 && (int)blockIdx.x + 1 == a.hold_cta1)) grid_arrive(a.grid_bar);
+        __syncthreads();   // the next tile is set up
+        drawn = false;
+        if (over) {
+            if (SH::PRE) {   // while the other CTAs arrive
+                draw_step<SH, 0>(tile<SH>().t, tile<SH>().d, tile<SH>().key);
+                drawn = true;
+            }
+            if (!grid_wait(a.grid_bar, gridDim.x * (uint32_t)so, a.wait_polls ? a.wait_polls : WAIT_POLLS)) {
+                if (tid == 0) atomicOr(a.error, 4u);
+                count_accepted(a.jobs[item.x].acc, accepted);
+                break;
+            }
         }
     }
-    }
-    if (!PER && a.nsteps > 1) grid_exit(a.grid_bar);
+    if (a.nsteps > 1) grid_exit(a.grid_bar);
 }
 
 }  // namespace elp
@@ -705,14 +885,12 @@ namespace {
 // Resident CTAs per SM of one kernel, per device (a cooperative launch is
 // sized by it); 0 until the group set-up on that device has asked.
 constexpr int MAX_DEVICES = 64;
-}
+using Kernel = void (*)(BatchLaunch);
 
-template <int TX, int TY, int TZ, bool PER, int NC, int SX, int SXY, int CAP, int K, int THREADS, int MINB, bool LIN>
-static cudaError_t launch2(const Sweep2Launch* l, cudaStream_t s)
+// Launch (or, with check_only, test) kernel k of shape SH.
+template <class SH, bool PER, int CAP, int MINB>
+cudaError_t launch2(const Sweep2Launch* l, Kernel k, std::atomic<int>* per_sm, cudaStream_t s)
 {
-    using SH = elp::Shape<TX, TY, TZ, PER, NC, SX, SXY, CAP, K, MINB>;
-    auto k = elp::sweep2_kernel<TX, TY, TZ, PER, NC, SX, SXY, CAP, K, THREADS, MINB, LIN>;
-    static std::atomic<int> per_sm[MAX_DEVICES];   // zero-initialised (static storage)
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -727,12 +905,12 @@ static cudaError_t launch2(const Sweep2Launch* l, cudaStream_t s)
         if (per_sm[dev].load() < 1) {
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::BYTES);
             int n = 0;
-            if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, THREADS, SH::BYTES);
+            if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, SH::THREADS, SH::BYTES);
             if (e != cudaSuccess) return e;
             if (n < 1) return cudaErrorNotSupported;
             per_sm[dev].store(n);
         }
-        const_cast<Sweep2Launch*>(l)->threads_out = THREADS;
+        const_cast<Sweep2Launch*>(l)->threads_out = SH::THREADS;
         const_cast<Sweep2Launch*>(l)->smem_out = SH::BYTES;
         return cudaSuccess;
     }
@@ -740,7 +918,7 @@ static cudaError_t launch2(const Sweep2Launch* l, cudaStream_t s)
     if (PER || l->args.nsteps <= 1) {
         if (grid > l->nsm * MINB) grid = l->nsm * MINB;
         if (grid < 1) return cudaSuccess;
-        k<<<grid, THREADS, SH::BYTES, s>>>(l->args);
+        k<<<grid, SH::THREADS, SH::BYTES, s>>>(l->args);
         return cudaGetLastError();
     }
     // tiled, several steps: a cooperative launch (every CTA resident, or an
@@ -751,7 +929,7 @@ static cudaError_t launch2(const Sweep2Launch* l, cudaStream_t s)
     if (grid < 1) return cudaSuccess;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(THREADS);
+    cfg.blockDim = dim3(SH::THREADS);
     cfg.dynamicSmemBytes = SH::BYTES;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -762,6 +940,23 @@ static cudaError_t launch2(const Sweep2Launch* l, cudaStream_t s)
     return cudaLaunchKernelEx(&cfg, k, l->args);
 }
 
+template <int TX, int NC, int SX, int SXY, int CAP, int K, bool LIN>
+cudaError_t launch_box(const Sweep2Launch* l, cudaStream_t s)
+{
+    static std::atomic<int> per_sm[MAX_DEVICES];   // zero-initialised (static storage)
+    return launch2<elp::Shape<TX, TX, TX, true, NC, SX, SXY, CAP, K, 1>, true, CAP, 1>(
+        l, elp::sweep_box<TX, NC, SX, SXY, CAP, K, LIN>, per_sm, s);
+}
+
+template <int TX, int TY, int TZ, int NC, int SX, int SXY, int CAP, int K, int MINB, bool LIN>
+cudaError_t launch_tiles(const Sweep2Launch* l, cudaStream_t s)
+{
+    static std::atomic<int> per_sm[MAX_DEVICES];
+    return launch2<elp::Shape<TX, TY, TZ, false, NC, SX, SXY, CAP, K, MINB>, false, CAP, MINB>(
+        l, elp::sweep_tiles<TX, TY, TZ, NC, SX, SXY, CAP, K, MINB, LIN>, per_sm, s);
+}
+}  // namespace
+
 // Launch (or, with check_only, test) the specialised kernel for a shape.
 // Returns cudaErrorNotSupported when none fits (the caller then uses the
 // generic kernel).
@@ -769,21 +964,26 @@ extern "C" cudaError_t elp_launch_sweep2(const Sweep2Launch* l, cudaStream_t s)
 {
     const elp_geometry& g = l->geom;
     if (l->args.nsteps > 1 && !g.periodic && !l->args.grid_bar) return cudaErrorNotSupported;
-// shape: tile edges, whole box or tiled, colour modulus, shared-memory
-// strides, slot capacity, anchors per thread, threads, min blocks per SM
-#define SHAPE(X_, Y_, Z_, PER_, NC_, SX_, SXY_, CAP_, K_, THR_, MINB_)                                        \
-    if (g.tx == X_ && g.ty == Y_ && g.tz == Z_ && g.periodic == PER_ && g.ncol == NC_ && l->sx == SX_ &&       \
-        l->sxy == SXY_)                                                                                        \
-        return l->linear ? launch2<X_, Y_, Z_, PER_, NC_, SX_, SXY_, CAP_, K_, THR_, MINB_, true>(l, s)        \
-                         : launch2<X_, Y_, Z_, PER_, NC_, SX_, SXY_, CAP_, K_, THR_, MINB_, false>(l, s);
-    SHAPE(32, 32, 32, 0, 16, 40, 1364, 1792, 2, 1024, 1)
-    SHAPE(32, 32, 16, 0, 16, 40, 1364, 1024, 1, 1024, 1)
-    SHAPE(32, 16, 16, 0, 16, 40, 724, 1024, 1, 512, 2)
-    SHAPE(16, 16, 16, 0, 16, 24, 444, 512, 1, 256, 4)
-    SHAPE(48, 24, 24, 0, 16, 56, 1456, 2048, 2, 864, 1)
-    SHAPE(16, 16, 16, 1, 16, 16, 256, 2048, 1, 256, 1)
-    SHAPE(32, 32, 32, 1, 16, 33, 1056, 2048, 2, 1024, 1)
-    SHAPE(24, 24, 24, 1, 24, 24, 576, 2048, 1, 576, 1)
-#undef SHAPE
+// tiles: edges, colour modulus, shared-memory strides, slot capacity, anchors
+// per thread, min blocks per SM
+#define TILES(X_, Y_, Z_, NC_, SX_, SXY_, CAP_, K_, MINB_)                                                      \
+    if (g.tx == X_ && g.ty == Y_ && g.tz == Z_ && !g.periodic && g.ncol == NC_ && l->sx == SX_ && l->sxy == SXY_) \
+        return l->linear ? launch_tiles<X_, Y_, Z_, NC_, SX_, SXY_, CAP_, K_, MINB_, true>(l, s)                \
+                         : launch_tiles<X_, Y_, Z_, NC_, SX_, SXY_, CAP_, K_, MINB_, false>(l, s);
+// whole boxes: edge, colour modulus, strides, slot capacity, anchors per thread
+#define BOX(X_, NC_, SX_, SXY_, CAP_, K_)                                                                       \
+    if (g.L == X_ && g.periodic && g.ncol == NC_ && l->sx == SX_ && l->sxy == SXY_)                             \
+        return l->linear ? launch_box<X_, NC_, SX_, SXY_, CAP_, K_, true>(l, s)                                 \
+                         : launch_box<X_, NC_, SX_, SXY_, CAP_, K_, false>(l, s);
+    TILES(32, 32, 32, 16, 40, 1364, 1792, 2, 1)
+    TILES(32, 32, 16, 16, 40, 1364, 1024, 1, 1)
+    TILES(32, 16, 16, 16, 40, 724, 1024, 1, 2)
+    TILES(16, 16, 16, 16, 24, 444, 512, 1, 3)
+    TILES(48, 24, 24, 16, 56, 1456, 2048, 2, 1)
+    BOX(16, 16, 16, 256, 2048, 1)
+    BOX(32, 16, 33, 1056, 2048, 2)
+    BOX(24, 24, 24, 576, 2048, 1)
+#undef BOX
+#undef TILES
     return cudaErrorNotSupported;
 }
