@@ -29,6 +29,7 @@ Sweep2Launch make_launch(const elp_group* G, int nsteps, uint32_t step_base, int
     l.args.jobs = G->d_jobs;
     l.args.items = G->d_items;
     l.args.nitems = G->nitems;
+    l.args.njobs = (int)G->jobs.size();
     l.args.nsteps = nsteps;
     l.args.step_base = step_base;
     l.args.step_dev = G->d_ctr;

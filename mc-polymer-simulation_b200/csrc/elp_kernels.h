@@ -45,7 +45,7 @@ struct BatchJob {
 struct BatchLaunch {
     const BatchJob* jobs;          // device job table
     const uint2* items;            // device work items {job, domain}
-    int nitems;
+    int nitems, njobs;             // (one job: item i is its domain i)
     int nsteps;                    // steps per launch
     uint32_t step_base;            // added to every job's step0 ...
     const uint32_t* step_dev;      // ... and, if set, this device counter (graph replays)

@@ -120,29 +120,34 @@ struct Shape {
     static constexpr int TABW = WORDS;
     static constexpr int OFFW = TABW + ELP_MOVE_ENTRIES;
     static constexpr int WOFFW = OFFW + NOFF;
+    static constexpr int TABS = WOFFW + (PER ? 0 : 16) - TABW;   // words of these tables
     static constexpr int COLW = (WOFFW + (PER ? 0 : 16) + 3) & ~3;
     static constexpr int NSLW = COLW + 4 * ((2 * NC + 3) / 4);   // slot count
-    static constexpr int TILEW = (NSLW + 4) & ~3;                // the tile at hand (Tile)
-    static constexpr int SCHW = TILEW + 16;
+    static constexpr int TILEW = (NSLW + 4) & ~3;                // the tile at hand and the next (Tile)
+    static constexpr int SCHW = TILEW + 2 * 20;
     static constexpr int SLOW = SCHW + CAP;
     static constexpr int HTABW = SLOW + CAP;  // table rows (0xf, x): moves of a linear chain's monomer 0
     static constexpr int RNDW = (HTABW + 64 + 3) & ~3;
     static constexpr int NSUB = 2 * NC;              // substeps per step
     static constexpr int NG = (NSUB + 3) / 4;        // groups of four substeps
-    // Random bytes, 16 per counter and group: in tiled domains, where MINB
-    // CTAs still fit on an SM (228 KB, 1 KB reserved per CTA), all NG groups
-    // of the step, drawn before its substeps (PRE); else one group's, read
-    // into registers as the group starts and overwritten with the next
-    // group's after its first barrier
-    static constexpr size_t bytes_with(int groups) { return (size_t)(RNDW + groups * A) * 4; }
-    static constexpr bool PRE = !PER && (size_t)MINB * (bytes_with(NG) + 1024) <= 233472;
-    static constexpr int TOTW = RNDW + (PRE ? NG : 1) * A;
+    // Random bytes, one word (four substeps) per anchor and group: in tiled
+    // domains, where MINB CTAs still fit on an SM (228 KB, 1 KB reserved per
+    // CTA), all NG groups of the step, drawn before its substeps (PRE); else
+    // one group's, read into registers as the group starts and overwritten
+    // with the next group's after its first barrier
+    static constexpr bool fits(int words) { return (size_t)MINB * ((size_t)words * 4 + 1024) <= 233472; }
+    static constexpr bool PRE = !PER && fits(RNDW + NG * A);
+    // where it fits too: a second table with each entry's change of the
+    // anchor's word (four instructions of a substep's 48)
+    static constexpr int DTABW = RNDW + (PRE ? NG : 1) * A;
+    static constexpr bool DT = fits(DTABW + ELP_MOVE_ENTRIES);
+    static constexpr int TOTW = DTABW + (DT ? ELP_MOVE_ENTRIES : 0);
     static constexpr size_t BYTES = (size_t)TOTW * 4;
     // neighbour offsets in words fit 16 signed bits (else they are taken
     // modulo 2^16, the reach of a shared-memory word index)
     static constexpr bool SOFF = !PER || (TX - 1) * (1 + SX + SXY) <= 32767;
     static_assert(A % 4 == 0 && A % K == 0 && THREADS <= 1024 && G <= THREADS, "anchors and draws per thread");
-    static_assert(K == 1 || (K == 2 && (A / 2) % G == 0), "the anchors of a thread share a Philox counter");
+    static_assert(K == 1 || K == 2, "anchors per thread");
     static_assert(CAP <= 2048, "slot numbers");
     static_assert(PER || (SX % 4 == 0 && SXY % 4 == 0 && SX >= SPAN + 1 && SXY >= SX * (TY + 2)),
                   "tiled rows: 16-byte aligned, room for the span and the halo word before it");
@@ -176,18 +181,6 @@ __device__ __forceinline__ void claim_slot(uint32_t wv, int idx)
     g_smem[SH::SCHW + slot] = wv >> 5;
     g_smem[SH::SLOW + slot] = (uint32_t)idx;   // until the record is fetched
 }
-// Fetch the chain record of each claimed slot: the word gets the slot number
-// and the run length, the slot monomer 0's offset.
-template <class SH>
-__device__ __forceinline__ void fill_slots(const uint32_t* rec, uint32_t ns)
-{
-    for (uint32_t sl = threadIdx.x; sl < ns; sl += SH::THREADS) {
-        const uint32_t idx = g_smem[SH::SLOW + sl];
-        const uint4 rr = __ldcg(reinterpret_cast<const uint4*>(rec + ELP_REC_WORDS * (size_t)g_smem[SH::SCHW + sl]));
-        g_smem[idx] = (g_smem[idx] & 15) | ((sl + 1) << SH::LSH) | (rr.y << ELP_CSHIFT);
-        g_smem[SH::SLOW + sl] = rr.z;
-    }
-}
 // A labelled word on its way out, from box site `site`: write the chain's
 // record and return the word's global form.
 template <class SH>
@@ -201,18 +194,22 @@ __device__ __forceinline__ uint32_t leave_slot(uint32_t wv, uint32_t site, uint3
 }
 
 // Monomer 0 sits in one of the runs an accepted move touched, whose new words
-// nP, nB, nY are stored (each with the label bits its old word had): bring its
-// slot number and offset to the run that holds it now.  Rarely needed; the
-// volatile accesses keep the compiler from folding it into the common case's
-// stores as selects that every move would pay for.
-template <class SH>
-__device__ __forceinline__ void follow_label(int p, int pB, int pY, uint32_t wP, uint32_t wB, uint32_t wY, bool s,
-                                             bool d1, bool join, uint32_t nP, uint32_t nB, uint32_t nY)
+// are stored (each with the label bits its old word had): bring its slot
+// number and offset to the run that holds it now.  Rarely needed, so it works
+// from what the move has in registers anyway and stores through volatile
+// accesses: otherwise the compiler computes its operands on every move, or
+// folds its stores into the move's own as selects (8 to 13 of 60 instructions
+// of every substep; now 3).
+template <class SH, bool PER>
+__device__ __forceinline__ void follow_label(int p, int pB, int pY, uint32_t wP, uint32_t wB, uint32_t wY, uint32_t R,
+                                             uint32_t E)
 {
     constexpr uint32_t LMASK = SH::LMASK;
     volatile uint32_t* const slot_off = g_smem + SH::SLOW - 1;
     volatile char* const S = reinterpret_cast<volatile char*>(g_smem);
     auto put = [&](int b, uint32_t w) { *reinterpret_cast<volatile uint32_t*>(S + b) = w; };
+    const bool s = (R & 0x8000u) != 0, d1 = PER ? (E >> 28) != 0 : ((int)E >> 18) != 0, join = (E & (15u << 9)) == 0;
+    const uint32_t nP = *reinterpret_cast<volatile uint32_t*>(S + p), nY = wY + ELP_CUNIT + ((E >> 9) & 15u);
     if (wP & LMASK) {
         // the anchor's run: monomer 0 leaves it as its last monomer only
         const uint32_t lb = wP & LMASK;
@@ -228,8 +225,8 @@ __device__ __forceinline__ void follow_label(int p, int pB, int pY, uint32_t wP,
         if (off0 > 0) {
             slot_off[lb >> SH::LSH] = off0 - 1;
         } else {
-            put(pB, nB & ~LMASK);
-            if (d1) put(pY, nY | lb);
+            put(pB, wB >= 2u * ELP_CUNIT ? (wB - ELP_CUNIT) & ~LMASK : 0u);
+            if (d1) put(pY, nY | lb);   // to the target, or to the end of P's run
             else put(p, nP | lb);
             slot_off[lb >> SH::LSH] = d1 ? 0u : (nP >> ELP_CSHIFT) - 1;
         }
@@ -241,20 +238,29 @@ __device__ __forceinline__ void follow_label(int p, int pB, int pY, uint32_t wP,
 
 // Random bytes of one substep group: byte q of words 0-3 of Philox counter
 // {t, d, group, gq} serves anchor gq + q G in the group's four substeps: bit
-// 0 the slot s, bits 1-4 the table option.  Kept with s in bit 7 and the
-// option in bits 2-5 of its byte: the slot then spreads over a byte by sign
-// replication and the option is a word offset.
-__device__ __forceinline__ uint4 draw_bytes(uint32_t t, int d, int group, int gq, uint2 key)
+// 0 the slot s, bits 1-4 the table option.  Kept as one word per anchor, a
+// byte per substep, with s in bit 7 and the option in bits 2-5: the slot then
+// spreads over a byte by sign replication and the option is a word offset.
+// (One 32-bit load per anchor and group; four words per counter took a
+// 128-bit load, 2 % more per step.)
+template <class SH>
+__device__ __forceinline__ void draw_bytes(uint32_t* r, uint32_t t, int d, int group, int gq, uint2 key)
 {
     uint4 v = philox(make_uint4(t, (uint32_t)d, (uint32_t)group, (uint32_t)gq), key);
     v.x = ((v.x << 7) & 0x80808080u) | ((v.x << 1) & 0x3C3C3C3Cu);
     v.y = ((v.y << 7) & 0x80808080u) | ((v.y << 1) & 0x3C3C3C3Cu);
     v.z = ((v.z << 7) & 0x80808080u) | ((v.z << 1) & 0x3C3C3C3Cu);
     v.w = ((v.w << 7) & 0x80808080u) | ((v.w << 1) & 0x3C3C3C3Cu);
-    return v;
+    const uint32_t xy01 = __byte_perm(v.x, v.y, 0x5140), zw01 = __byte_perm(v.z, v.w, 0x5140);
+    const uint32_t xy23 = __byte_perm(v.x, v.y, 0x7362), zw23 = __byte_perm(v.z, v.w, 0x7362);
+    r[gq] = __byte_perm(xy01, zw01, 0x5410);
+    r[gq + SH::G] = __byte_perm(xy01, zw01, 0x7632);
+    r[gq + 2 * SH::G] = __byte_perm(xy23, zw23, 0x5410);
+    r[gq + 3 * SH::G] = __byte_perm(xy23, zw23, 0x7632);
 }
+// Group g's words (one buffer unless PRE).
 template <class SH>
-__device__ __forceinline__ uint4* random_words() { return reinterpret_cast<uint4*>(g_smem + SH::RNDW); }
+__device__ __forceinline__ uint32_t* random_words(int g) { return g_smem + SH::RNDW + (SH::PRE ? g * SH::A : 0); }
 
 // All groups of a step (PRE), in two parts.
 template <class SH, int PART>
@@ -262,18 +268,18 @@ __device__ __forceinline__ void draw_step(uint32_t t, int d, uint2 key)
 {
     constexpr int N = SH::NG * SH::G, H = (N / SH::THREADS + 1) / 2 * SH::THREADS;
     for (int i = threadIdx.x + (PART ? H : 0); i < (PART ? N : (H < N ? H : N)); i += SH::THREADS)
-        random_words<SH>()[i] = draw_bytes(t, d, i / SH::G, i % SH::G, key);
+        draw_bytes<SH>(random_words<SH>(i / SH::G), t, d, i / SH::G, i % SH::G, key);
 }
 
-// The byte that selector sel names (byte_selector) as the low byte, its top
-// bit spread over the next byte, zeros above.
-__device__ __forceinline__ uint32_t spread_byte(uint32_t w, uint32_t sel)
+// Byte kk of a random word as the low byte, its top bit spread over the next
+// byte, zeros above.
+template <int KK>
+__device__ __forceinline__ uint32_t spread_byte(uint32_t w)
 {
     uint32_t r;
-    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(w), "r"(sel));
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(w), "n"(0x4400 | (8 | KK) << 4 | KK));
     return r;
 }
-__device__ __forceinline__ uint32_t byte_selector(uint32_t q) { return 0x4400u | (8u | q) << 4 | q; }
 
 // The step's colours, in bytes of x offset, drawn by one warp of the CTA;
 // lane 31 returns the words of the step's domain shift.
@@ -298,22 +304,23 @@ struct Tile {
     uint32_t t;         // absolute step
     int d, L;           // domain, box edge
     int x0, y0, z0;     // box site of the tile's first word
+    unsigned long long* acc;
 };
-static_assert(sizeof(Tile) <= 64, "16 words of shared memory");
+static_assert(sizeof(Tile) <= 80, "20 words of shared memory");
+// The tile at hand and the next one are slots par and par ^ 1.
 template <class SH>
-__device__ __forceinline__ Tile& tile() { return *reinterpret_cast<Tile*>(g_smem + SH::TILEW); }
+__device__ __forceinline__ Tile& tile(int par) { return *reinterpret_cast<Tile*>(g_smem + SH::TILEW + 20 * par); }
 
-// Set up the next tile (one warp): item it of the launch at its step so.
+// Set up a tile (one warp): domain item.y of melt J at `step`.
 template <class SH, int TX, int TY, int TZ, int NC>
-__device__ __forceinline__ void next_tile(const BatchLaunch& a, uint2 item, uint32_t step)
+__device__ __forceinline__ void set_tile(const BatchJob& J, int d, uint32_t step, int par)
 {
-    const BatchJob& J = a.jobs[item.x];
-    const int d = (int)item.y, ntx = J.ntx, nty = J.nty;
+    const int ntx = J.ntx, nty = J.nty;
     const uint32_t t = J.step0 + step;
     const uint2 key = make_uint2(J.seed, J.salt);
     const uint4 w = draw_schedule<SH, NC>(t, d, key);
     if ((threadIdx.x & 31) == 31) {
-        Tile& T = tile<SH>();
+        Tile& T = tile<SH>(par);
         T.lat = J.lat;
         T.rec = J.rec;
         T.key = key;
@@ -323,7 +330,26 @@ __device__ __forceinline__ void next_tile(const BatchLaunch& a, uint2 item, uint
         T.x0 = (int)bounded(w.x, TX) + (d % ntx) * TX;
         T.y0 = (int)bounded(w.y, TY) + ((d / ntx) % nty) * TY;
         T.z0 = (int)bounded(w.z, TZ) + (d / ntx / nty) * TZ;
+        T.acc = J.acc;
         g_smem[SH::NSLW] = 0;
+    }
+}
+
+// Fetch the chain record of each claimed slot: the word gets the slot number
+// and the run length, the slot monomer 0's offset.  A tile's other random
+// bytes (PRE) are drawn while the records are on their way.
+template <class SH>
+__device__ __forceinline__ void fill_slots(const Tile& T, uint32_t ns)
+{
+    const uint32_t tid = threadIdx.x;
+    uint4 rr = make_uint4(0, 0, 0, 0);
+    if (tid < ns) rr = __ldcg(reinterpret_cast<const uint4*>(T.rec + ELP_REC_WORDS * (size_t)g_smem[SH::SCHW + tid]));
+    if (SH::PRE) draw_step<SH, 1>(T.t, T.d, T.key);
+    for (uint32_t sl = tid; sl < ns; sl += SH::THREADS) {
+        if (sl != tid) rr = __ldcg(reinterpret_cast<const uint4*>(T.rec + ELP_REC_WORDS * (size_t)g_smem[SH::SCHW + sl]));
+        const uint32_t idx = g_smem[SH::SLOW + sl];
+        g_smem[idx] = (g_smem[idx] & 15) | ((sl + 1) << SH::LSH) | (rr.y << ELP_CSHIFT);
+        g_smem[SH::SLOW + sl] = rr.z;
     }
 }
 
@@ -343,8 +369,6 @@ __device__ __forceinline__ int fresh_tid()
 template <int K>
 struct Anchors {
     int base[K], rot[K], cls[K], xlo[K], xhi[K], an[K];
-    uint32_t sel[K];   // byte of the counter's words
-    int gq;            // the counter they share
 };
 // Anchor an = g + q G of a substep takes byte q of Philox counter g.  Thread
 // tid owns anchors an = tid + q AT, or with PERM the anchors of the same x
@@ -359,12 +383,10 @@ __device__ __forceinline__ void set_anchors(Anchors<K>& o)
         const int y = (lane & 7) + 8 * (w % (TY / 8)), z = (lane >> 3) + 4 * (w / (TY / 8));
         tperm = tid - r + y + TY * z;
     }
-    o.gq = tperm % SH::G;
 #pragma unroll
     for (int q = 0; q < K; q++) {
         const int an = tperm + q * SH::AT;
         o.an[q] = an;
-        o.sel[q] = byte_selector((uint32_t)(an / SH::G));
         const int j = an / SH::R, row = an % SH::R;
         const int y = row % TY, z = row / TY;
         const int m = (2 * y + 3 * z) % NC;
@@ -396,26 +418,26 @@ __device__ __forceinline__ int colour_x(int c4, int rot)
 // The anchors are passed by value so that the caller's copies stay in
 // registers.
 template <class SH, int K, int NC, int SX, int SXY>
-__device__ __noinline__ uint32_t general_substeps(const Anchors<K> an, const uint8_t* table)
+__device__ __noinline__ uint32_t general_substeps(const Anchors<K> an, const uint8_t* table, int par)
 {
     const int* woffs = reinterpret_cast<const int*>(g_smem + SH::WOFFW);
-    const Tile T = tile<SH>();
+    const Tile T = tile<SH>(par);
     const int sh4 = 4 * (T.x0 & 3);
     Dom D;
     D.S = g_smem; D.tab = table; D.rec = T.rec;
     D.ox = SH::OX + (T.x0 & 3); D.sx = SX; D.sxy = SXY; D.L = T.L;
     D.x0 = T.x0; D.y0 = T.y0; D.z0 = T.z0;
-    uint4* rnd = random_words<SH>();
     uint32_t acc = 0;
     for (int g = 0; g < SH::NG; g++) {
-        const uint4 v = rnd[(SH::PRE ? g * SH::G : 0) + an.gq];
+        uint32_t rw[K];
+        for (int q = 0; q < K; q++) rw[q] = random_words<SH>(g)[an.an[q]];
         for (int kk = 0; kk < 4 && 4 * g + kk < SH::NSUB; kk++) {
             const int c4 = (int)g_smem[SH::COLW + 4 * g + kk];
             if (!SH::PRE && kk == 1 && (int)threadIdx.x < SH::G && g + 1 < SH::NG)
-                rnd[threadIdx.x] = draw_bytes(T.t, T.d, g + 1, (int)threadIdx.x, T.key);
+                draw_bytes<SH>(random_words<SH>(g + 1), T.t, T.d, g + 1, (int)threadIdx.x, T.key);
             for (int q = 0; q < K; q++) {
                 const int xr4 = colour_x<NC>(c4, an.rot[q]);
-                const uint32_t b = spread_byte(word_of(v, kk), an.sel[q]);
+                const uint32_t b = rw[q] >> (8 * kk);
                 if (!SH::TAIL || (int)threadIdx.x < SH::AT)
                     acc += (uint32_t)op(D, (an.base[q] + sh4 + xr4) >> 2, woffs, ((b >> 7) & 1u) | ((b >> 1) & 0x1Eu));
             }
@@ -425,8 +447,8 @@ __device__ __noinline__ uint32_t general_substeps(const Anchors<K> an, const uin
     return acc;
 }
 
-// The K anchors of one thread, one substep, random bytes in word w.  Returns
-// accepted moves.  c4 = 4 c, k the substep; LIN: the melt holds linear chains
+// The K anchors of one thread, one substep, random bytes in byte KK of words
+// rw.  Returns accepted moves.  c4 = 4 c, k the substep; LIN: the melt holds linear chains
 // (head moves of monomer 0).
 //
 // The kernel is bound by instruction issue and shared-memory wavefronts, so
@@ -436,9 +458,9 @@ __device__ __noinline__ uint32_t general_substeps(const Anchors<K> an, const uin
 // from additions, and the target and next run are stored ahead of the anchor
 // so that a move back into the anchor's run (target = anchor) needs no case
 // of its own.
-template <class SH, int K, bool PER, int NC, bool LIN>
-__device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, uint32_t w, uint32_t voff, int c4, uint32_t t,
-                                             int d, int k, uint2 key)
+template <class SH, int K, bool PER, int NC, bool LIN, int KK>
+__device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, const uint32_t (&rw)[K], uint32_t voff, int c4,
+                                             uint32_t t, int d, int k, uint2 key)
 {
     constexpr int TAB4 = 4 * SH::TABW;
     int p[K], tc[K];
@@ -448,8 +470,8 @@ __device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, uint
         const int xr4 = colour_x<NC>(c4, an.rot[q]);
         p[q] = an.base[q] + sh4 + xr4;
         wP[q] = SW(p[q]);
-        if (SH::TAIL && (int)threadIdx.x >= SH::AT) wP[q] = 0;   // an empty site: no move
-        R[q] = spread_byte(w, an.sel[q]);
+        R[q] = spread_byte<KK>(rw[q]);
+        if (SH::TAIL && (int)threadIdx.x >= SH::AT) wP[q] = R[q] = 0;   // slot 0 of an empty site: no move
         // whole box: the boundary class's offsets (64 bytes each)
         tc[q] = PER ? an.cls[q] + (xr4 == an.xlo[q] ? -64 : 0) + (xr4 == an.xhi[q] ? 64 : 0) : 0;
     }
@@ -465,7 +487,7 @@ __device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, uint
         const uint32_t w1 = SW(pB[q]);
         wB[q] = (R[q] & 0x8000u) ? w1 : wP[q];
     }
-    uint32_t E[K];
+    uint32_t E[K], D[K];
     bool c2[K];
 #pragma unroll
     for (int q = 0; q < K; q++) {
@@ -476,6 +498,7 @@ __device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, uint
         uint32_t ix = R[q] & (V[q] | 0x3Cu);
         if (c2[q] != s) ix += (wB[q] & 15) << 6;
         E[q] = SW(TAB4 + (int)ix);
+        if (SH::DT) D[q] = SW(4 * SH::DTABW + (int)ix);
     }
     int pY[K];
     uint32_t wY[K];
@@ -494,20 +517,15 @@ __device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, uint
     for (int q = 0; q < K; q++) {
         const bool s = (R[q] & 0x8000u) != 0;
         const bool ok = E[q] != 0 && (wY[q] & E[q] & (PER ? 0xFu : 0x1Fu)) == 0;
-        const uint32_t nP = ((wP[q] & ~15u) | ((E[q] >> 5) & 15u)) + (E[q] & 0x30000u) - ELP_CUNIT;
+        const uint32_t nP = SH::DT ? wP[q] + D[q]
+                                   : ((wP[q] & ~15u) | ((E[q] >> 5) & 15u)) + (E[q] & 0x30000u) - ELP_CUNIT;
         const uint32_t nB = c2[q] ? wB[q] - ELP_CUNIT : 0u;
         const uint32_t nY = wY[q] + ELP_CUNIT + ((E[q] >> 9) & 15u);
         if (ok) SW(pY[q]) = nY;
         if (ok && s) SW(pB[q]) = nB;
         if (ok) SW(p[q]) = nP;
         const bool lab = ok && ((wP[q] | wB[q] | wY[q]) & SH::LMASK);
-        // a branch of the whole warp: predicated, its instructions would be
-        // issued on every substep
-        if (__any_sync(0xffffffffu, lab)) {
-            const bool d1 = PER ? (E[q] >> 28) != 0 : ((int)E[q] >> 18) != 0;
-            if (lab)
-                follow_label<SH>(p[q], pB[q], pY[q], wP[q], wB[q], wY[q], s, d1, (E[q] & (15u << 9)) == 0, nP, nB, nY);
-        }
+        if (lab) follow_label<SH, PER>(p[q], pB[q], pY[q], wP[q], wB[q], wY[q], R[q], E[q]);
         if (LIN && ok) wP[q] = lab ? SW(p[q]) : nP;
         acc += ok ? 1u : 0u;
     }
@@ -550,34 +568,35 @@ __device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, uint
 
 // The substeps of one step of a domain.  Returns this thread's accepted moves.
 template <class SH, int K, bool PER, int NC, bool LIN>
-__device__ __forceinline__ uint32_t substeps(const Anchors<K>& an, int sh4, uint32_t voff)
+__device__ __forceinline__ uint32_t substeps(const Anchors<K>& an, int sh4, uint32_t voff, int par)
 {
-    uint4* rnd = random_words<SH>();
     uint32_t acc = 0;
     // what draws need in here (linear chains; groups drawn one at a time)
     uint32_t t = 0;
     int d = 0;
     uint2 key = make_uint2(0, 0);
     if (LIN || !SH::PRE) {
-        t = tile<SH>().t;
-        d = tile<SH>().d;
-        key = tile<SH>().key;
+        t = tile<SH>(par).t;
+        d = tile<SH>(par).d;
+        key = tile<SH>(par).key;
     }
 #pragma unroll 1
     for (int g = 0; g < SH::NG; g++) {
         const uint4 c4 = reinterpret_cast<const uint4*>(g_smem + SH::COLW)[g];
-        const uint4 v = rnd[(SH::PRE ? g * SH::G : 0) + an.gq];
-        acc += substepK<SH, K, PER, NC, LIN>(an, sh4, v.x, voff, (int)c4.x, t, d, 4 * g, key);
+        uint32_t rw[K];
+#pragma unroll
+        for (int q = 0; q < K; q++) rw[q] = random_words<SH>(g)[an.an[q]];
+        acc += substepK<SH, K, PER, NC, LIN, 0>(an, sh4, rw, voff, (int)c4.x, t, d, 4 * g, key);
         __syncthreads();
         // the next group's bytes: every thread has read this group's
         if (!SH::PRE && (int)threadIdx.x < SH::G && g + 1 < SH::NG)
-            rnd[threadIdx.x] = draw_bytes(t, d, g + 1, (int)threadIdx.x, key);
-        acc += substepK<SH, K, PER, NC, LIN>(an, sh4, v.y, voff, (int)c4.y, t, d, 4 * g + 1, key);
+            draw_bytes<SH>(random_words<SH>(g + 1), t, d, g + 1, (int)threadIdx.x, key);
+        acc += substepK<SH, K, PER, NC, LIN, 1>(an, sh4, rw, voff, (int)c4.y, t, d, 4 * g + 1, key);
         __syncthreads();
         if (SH::NSUB % 4 && 4 * g + 2 >= SH::NSUB) break;
-        acc += substepK<SH, K, PER, NC, LIN>(an, sh4, v.z, voff, (int)c4.z, t, d, 4 * g + 2, key);
+        acc += substepK<SH, K, PER, NC, LIN, 2>(an, sh4, rw, voff, (int)c4.z, t, d, 4 * g + 2, key);
         __syncthreads();
-        acc += substepK<SH, K, PER, NC, LIN>(an, sh4, v.w, voff, (int)c4.w, t, d, 4 * g + 3, key);
+        acc += substepK<SH, K, PER, NC, LIN, 3>(an, sh4, rw, voff, (int)c4.w, t, d, 4 * g + 3, key);
         __syncthreads();
     }
     return acc;
@@ -591,14 +610,17 @@ __device__ __forceinline__ void count_accepted(unsigned long long* acc, unsigned
     if ((threadIdx.x & 31) == 0 && v) atomicAdd(acc, v);
 }
 
-// Tables of a launch into shared memory: moves and neighbour offsets
-// (elp_move_table builds them in this order) and rows (0xf, x) of the
+// Tables of a launch into shared memory: moves, neighbour offsets, changes of
+// the anchor's word (elp_move_table builds them in this order) and rows (0xf, x) of the
 // transition table (moves of a linear chain's monomer 0).
 template <class SH, bool PER>
 __device__ __forceinline__ void load_tables(const BatchLaunch& a)
 {
-    for (int i = threadIdx.x; i < (ELP_MOVE_ENTRIES + SH::NOFF + (PER ? 0 : 16)) / 4; i += SH::THREADS)
-        cp_async16(g_smem + SH::TABW + 4 * i, a.moves + 4 * i);
+    static_assert(SH::TABS % 4 == 0 && SH::TABW % 4 == 0 && SH::DTABW % 4 == 0, "16-byte copies");
+    for (int i = threadIdx.x; i < SH::TABS / 4; i += SH::THREADS) cp_async16(g_smem + SH::TABW + 4 * i, a.moves + 4 * i);
+    if (SH::DT)
+        for (int i = threadIdx.x; i < ELP_MOVE_ENTRIES / 4; i += SH::THREADS)
+            cp_async16(g_smem + SH::DTABW + 4 * i, a.moves + SH::TABS + 4 * i);
     for (int i = threadIdx.x; i < 64; i += SH::THREADS) g_smem[SH::HTABW + i] = a.table[960 + i];
 }
 
@@ -641,19 +663,21 @@ __global__ void __launch_bounds__(((TX * TX * (TX / NC) / K) + 31) / 32 * 32, 1)
             if (tid == 0) atomicOr(a.error, 1u);
             continue;
         }
-        fill_slots<SH>(rec, ns);
+        if (tid == 0) tile<SH>(0).rec = rec;
+        __syncthreads();
+        fill_slots<SH>(tile<SH>(0), ns);
         unsigned long long accepted = 0;
         for (int st = 0; st < a.nsteps; st++) {
             const uint32_t t = t0 + (uint32_t)st;
-            if (tid < SH::G) random_words<SH>()[tid] = draw_bytes(t, 0, 0, tid, key);
+            if (tid < SH::G) draw_bytes<SH>(random_words<SH>(0), t, 0, 0, tid, key);
             if (tid >= SH::THREADS - 32) draw_schedule<SH, NC>(t, 0, key);
             if (tid == 0) {
-                tile<SH>().t = t;
-                tile<SH>().d = 0;
-                tile<SH>().key = key;
+                tile<SH>(0).t = t;
+                tile<SH>(0).d = 0;
+                tile<SH>(0).key = key;
             }
             __syncthreads();
-            accepted += substeps<SH, K, true, NC, LIN>(an, 0, 0u);
+            accepted += substeps<SH, K, true, NC, LIN>(an, 0, 0u, 0);
         }
         for (int i = tid; i < SITES; i += SH::THREADS) {
             uint32_t wv = S[i % TX + SX * (i / TX % TX) + SXY * (i / (TX * TX))];
@@ -692,16 +716,22 @@ __global__ void __launch_bounds__(((TY * TZ * (TX / NC) / K) + 31) / 32 * 32, MI
     const bool scheduler = tid >= SH::THREADS - 32;   // the warp that sets up the next tile
     const uint32_t step0 = a.step_base + (a.step_dev ? *a.step_dev : 0u);
 
-    uint2 item = a.items[blockIdx.x];
     unsigned long long accepted = 0;
-    bool drawn = false;   // the first part of the tile's random bytes is on chip already
-    if (scheduler) next_tile<SH, TX, TY, TZ, NC>(a, item, step0);
+    int par = 0;
+    // one melt alone: its job stays in registers of the warp that needs it
+    const bool alone = a.njobs == 1;
+    BatchJob J;
+    if (scheduler) {
+        const uint2 item = alone ? make_uint2(0u, blockIdx.x) : a.items[blockIdx.x];
+        J = a.jobs[item.x];
+        set_tile<SH, TX, TY, TZ, NC>(J, (int)item.y, step0, 0);
+    }
     __syncthreads();
     for (int so = 0, it = blockIdx.x;;) {
         // ---- load: quads of four words; a quad never straddles x = L (L and
         // xa are multiples of 4)
         {
-            const Tile T = tile<SH>();
+            const Tile T = tile<SH>(par);
             const int ft = fresh_tid(), L = T.L;
             const bool mover = !SH::TAIL || ft < SH::AT, ender = SH::R == SH::THREADS || ft < SH::R;
             const uint32_t LL = (uint32_t)(L * L);
@@ -730,10 +760,8 @@ __global__ void __launch_bounds__(((TY * TZ * (TX / NC) / K) + 31) / 32 * 32, MI
                     if (mover) v[i] = __ldcg(reinterpret_cast<const uint4*>(src + LL * (uint32_t)z));
                     z += SH::ZS; z -= z >= L ? L : 0;
                 }
-                if (SH::PRE && i0 == 0) {   // the step's random bytes while the quads are on their way
-                    if (!drawn) draw_step<SH, 0>(T.t, T.d, T.key);
-                    draw_step<SH, 1>(T.t, T.d, T.key);
-                }
+                // half of the step's random bytes while the quads are on their way
+                if (SH::PRE && i0 == 0) draw_step<SH, 0>(T.t, T.d, T.key);
 #pragma unroll
                 for (int i = 0; i < NB; i++) {
                     if (mc == 0) {   // words ahead of the tile
@@ -761,7 +789,7 @@ __global__ void __launch_bounds__(((TY * TZ * (TX / NC) / K) + 31) / 32 * 32, MI
                 ve.w = HWALL;
                 *reinterpret_cast<uint4*>(S + at) = ve;
             }
-            if (!SH::PRE && tid < SH::G) random_words<SH>()[tid] = draw_bytes(T.t, T.d, 0, tid, T.key);
+            if (!SH::PRE && tid < SH::G) draw_bytes<SH>(random_words<SH>(0), T.t, T.d, 0, tid, T.key);
         }
         __syncthreads();
 
@@ -769,9 +797,9 @@ __global__ void __launch_bounds__(((TY * TZ * (TX / NC) / K) + 31) / 32 * 32, MI
         const uint32_t ns = g_smem[SH::NSLW];
         const bool crowded = ns > (uint32_t)SH::SLOTS;
         if (!crowded) {
-            fill_slots<SH>(tile<SH>().rec, ns);
+            fill_slots<SH>(tile<SH>(par), ns);
             __syncthreads();
-            accepted += substeps<SH, K, false, NC, LIN>(an, 4 * (tile<SH>().x0 & 3), voff);
+            accepted += substeps<SH, K, false, NC, LIN>(an, 4 * (tile<SH>(par).x0 & 3), voff, par);
         } else if (!LIN) {
             // a crowded ring tile: its words are still in their global form
             // and the records hold the runs' lengths and offsets; halo words
@@ -779,19 +807,22 @@ __global__ void __launch_bounds__(((TY * TZ * (TX / NC) / K) + 31) / 32 * 32, MI
             for (int i = tid; i < SH::WORDS; i += SH::THREADS)
                 if (S[i] == HWALL) S[i] = ELP_WALL;
             __syncthreads();
-            accepted += general_substeps<SH, K, NC, SX, SXY>(an, reinterpret_cast<const uint8_t*>(a.table));
+            if (SH::PRE) draw_step<SH, 1>(tile<SH>(par).t, tile<SH>(par).d, tile<SH>(par).key);
+            __syncthreads();
+            accepted += general_substeps<SH, K, NC, SX, SXY>(an, reinterpret_cast<const uint8_t*>(a.table), par);
             for (int i = tid; i < SH::WORDS; i += SH::THREADS)
                 if (S[i] == ELP_WALL) S[i] = HWALL;
             __syncthreads();
-        } else if (tid == 0) {
+        } else {
             // linear chains: the general move does not apply; leave the tile
             // untouched, report
-            atomicOr(a.error, 1u);
+            if (tid == 0) atomicOr(a.error, 1u);
+            __syncthreads();   // every thread has read the count
         }
 
         // ---- store: quads inside the tile, single words at its ragged ends
         if (!crowded || !LIN) {
-            const Tile T = tile<SH>();
+            const Tile T = tile<SH>(par);
             const int ft = fresh_tid(), L = T.L;
             const bool mover = !SH::TAIL || ft < SH::AT, ender = SH::R == SH::THREADS || ft < SH::R;
             const uint32_t LL = (uint32_t)(L * L), lmask = crowded ? 0u : SH::LMASK;
@@ -849,28 +880,28 @@ __global__ void __launch_bounds__(((TY * TZ * (TX / NC) / K) + 31) / 32 * 32, MI
             it = blockIdx.x;
             so++;
         }
-        const bool last = so >= a.nsteps;
-        const uint32_t job = item.x;
-        if (!last) item = a.items[it];
-        if (last || item.x != job) {
-            count_accepted(a.jobs[job].acc, accepted);
+        if (so >= a.nsteps) {
+            count_accepted(tile<SH>(par).acc, accepted);
+            break;
+        }
+        if (scheduler) {
+            const uint2 item = alone ? make_uint2(0u, (uint32_t)it) : a.items[it];
+            if (!alone) J = a.jobs[item.x];
+            set_tile<SH, TX, TY, TZ, NC>(J, (int)item.y, step0 + (uint32_t)so, par ^ 1);
+        }
+        __syncthreads();   // the tile's words have been read, the next tile is set up
+        unsigned long long* const acc = tile<SH>(par).acc;
+        par ^= 1;
+        if (acc != tile<SH>(par).acc) {
+            count_accepted(acc, accepted);
             accepted = 0;
         }
-        if (last) break;
-        __syncthreads();   // the tile's words and description have been read
-        if (scheduler) next_tile<SH, TX, TY, TZ, NC>(a, item, step0 + (uint32_t)so);
-        // a test may keep one CTA from arriving at the first barrier
-        if (over && tid == 0 && !(so == 1 && (int)blockIdx.x + 1 == a.hold_cta1)) grid_arrive(a.grid_bar);
-        __syncthreads();   // the next tile is set up
-        drawn = false;
         if (over) {
-            if (SH::PRE) {   // while the other CTAs arrive
-                draw_step<SH, 0>(tile<SH>().t, tile<SH>().d, tile<SH>().key);
-                drawn = true;
-            }
+            // a test may keep one CTA from arriving at the first barrier
+            if (tid == 0 && !(so == 1 && (int)blockIdx.x + 1 == a.hold_cta1)) grid_arrive(a.grid_bar);
             if (!grid_wait(a.grid_bar, gridDim.x * (uint32_t)so, a.wait_polls ? a.wait_polls : WAIT_POLLS)) {
                 if (tid == 0) atomicOr(a.error, 4u);
-                count_accepted(a.jobs[item.x].acc, accepted);
+                count_accepted(tile<SH>(par).acc, accepted);
                 break;
             }
         }
@@ -983,6 +1014,28 @@ extern "C" cudaError_t elp_launch_sweep2(const Sweep2Launch* l, cudaStream_t s)
     BOX(16, 16, 16, 256, 2048, 1)
     BOX(32, 16, 33, 1056, 2048, 2)
     BOX(24, 24, 24, 576, 2048, 1)
+#undef BOX
+#undef TILES
+// Shapes of rings only (linear chains of these boxes are refused): the even
+// boxes between, and the tiles that boxes of 40, 60, 72, 100, 120 ... take.
+// On the generic kernel their steps took 171 us (L = 20), 175 (28), 238 (40)
+// and 251 (72); @20@ here.
+#define TILES(X_, Y_, Z_, NC_, SX_, SXY_, CAP_, K_, MINB_)                                                       \
+    if (g.tx == X_ && g.ty == Y_ && g.tz == Z_ && !g.periodic && g.ncol == NC_ && l->sx == SX_ &&                \
+        l->sxy == SXY_ && !l->linear)                                                                            \
+        return launch_tiles<X_, Y_, Z_, NC_, SX_, SXY_, CAP_, K_, MINB_, false>(l, s);
+#define BOX(X_, NC_, SX_, SXY_, CAP_, K_)                                                                       \
+    if (g.L == X_ && g.periodic && g.ncol == NC_ && l->sx == SX_ && l->sxy == SXY_ && !l->linear)               \
+        return launch_box<X_, NC_, SX_, SXY_, CAP_, K_, false>(l, s);
+    TILES(24, 24, 24, 24, 32, 832, 2048, 1, 1)
+    TILES(40, 20, 20, 20, 48, 1056, 2048, 1, 1)
+    TILES(20, 20, 20, 20, 28, 616, 1024, 1, 2)
+    BOX(18, 18, 20, 360, 2048, 1)
+    BOX(20, 20, 21, 422, 2048, 1)
+    BOX(22, 22, 22, 484, 2048, 1)
+    BOX(26, 13, 26, 676, 2048, 2)
+    BOX(28, 14, 30, 840, 2048, 2)
+    BOX(30, 15, 30, 900, 2048, 2)
 #undef BOX
 #undef TILES
     return cudaErrorNotSupported;
