@@ -448,16 +448,20 @@ __device__ __noinline__ uint32_t general_substeps(const Anchors<K> an, const uin
 }
 
 // The K anchors of one thread, one substep, random bytes in byte KK of words
-// rw.  Returns accepted moves.  c4 = 4 c, k the substep; LIN: the melt holds linear chains
-// (head moves of monomer 0).
+// rw.  Returns accepted moves.  c4 = 4 c, k the substep; LIN: the melt holds
+// linear chains (head moves of monomer 0).
 //
-// The kernel is bound by instruction issue and shared-memory wavefronts, so
-// the move is written for few instructions (49 per warp and substep, 72
-// before; L = 256: 145.8 -> 126 us per step with the tile copy below): one 32-bit entry of the move table carries everything the
-// move's rows decide (target, test, the new words' parts), new words come
-// from additions, and the target and next run are stored ahead of the anchor
-// so that a move back into the anchor's run (target = anchor) needs no case
-// of its own.
+// The kernel is bound by instruction issue (the ALU pipe takes an instruction
+// every other cycle) and by the chain of shared-memory loads, so the move is
+// written for few instructions: 43 per warp and substep, 21 of them on the
+// ALU pipe (the move of elp_device.cuh laid out the same way: 81 and 40).
+// One 32-bit entry of the move table carries everything the move's rows
+// decide (target, test, the new words' parts), new words come from additions,
+// and the target and next run are stored ahead of the anchor so that a move
+// back into the anchor's run (target = anchor) needs no case of its own.
+// L = 256: 145.8 -> 113.6 us per step together with the tile copy below.
+// Loads predicated on the lanes that need them cut a tenth of the
+// shared-memory wavefronts but were 3 % slower.
 template <class SH, int K, bool PER, int NC, bool LIN, int KK>
 __device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, const uint32_t (&rw)[K], uint32_t voff, int c4,
                                              uint32_t t, int d, int k, uint2 key)
@@ -695,10 +699,11 @@ __global__ void __launch_bounds__(((TX * TX * (TX / NC) / K) + 31) / 32 * 32, 1)
 // of a step's 23.2 us, mostly address arithmetic (1180 instructions per warp,
 // now 790) and latencies in a row.  So a thread's quads differ by whole planes
 // only, labelled words are found in registers on the way in and out, the
-// step's random bytes are drawn while the quads are on their way and between
-// arriving at the grid barrier and waiting for it, and what a tile's load and
-// store need sits in shared memory in between (held in registers it made the
-// substep loop recompute its own).  19.4 us per step now, 23.4 before.
+// step's random bytes are drawn while the quads and the chain records are on
+// their way, the next tile is set up while this one is stored, and what a
+// tile's load and store need sits in shared memory in between (held in
+// registers it made the substep loop recompute its own).  18.4 us per step
+// now, 23.4 before.
 template <int TX, int TY, int TZ, int NC, int SX, int SXY, int CAP, int K, int MINB, bool LIN>
 __global__ void __launch_bounds__(((TY * TZ * (TX / NC) / K) + 31) / 32 * 32, MINB) sweep_tiles(BatchLaunch a)
 {
@@ -1018,8 +1023,8 @@ extern "C" cudaError_t elp_launch_sweep2(const Sweep2Launch* l, cudaStream_t s)
 #undef TILES
 // Shapes of rings only (linear chains of these boxes are refused): the even
 // boxes between, and the tiles that boxes of 40, 60, 72, 100, 120 ... take.
-// On the generic kernel their steps took 171 us (L = 20), 175 (28), 238 (40)
-// and 251 (72); @20@ here.
+// On the generic kernel a step took 171 us (L = 20), 175 (28), 238 (40) and
+// 251 (72); here 14.9, 24.4, 23.5 and 21.7.
 #define TILES(X_, Y_, Z_, NC_, SX_, SXY_, CAP_, K_, MINB_)                                                       \
     if (g.tx == X_ && g.ty == Y_ && g.tz == Z_ && !g.periodic && g.ncol == NC_ && l->sx == SX_ &&                \
         l->sxy == SXY_ && !l->linear)                                                                            \
