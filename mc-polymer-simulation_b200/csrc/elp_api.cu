@@ -262,12 +262,11 @@ extern "C" elp_status elp_fetch_chains(elp_ctx* c, int32_t* start, uint8_t* bond
     if (!c || !start || !bonds) return elp_fail(ELP_ERR_ARG, "null argument");
     if (!c->loaded) return elp_fail(ELP_ERR_STATE, "no configuration loaded");
     ELP_CUDA_TRY(cudaSetDevice(c->device));
-    // the walk is queued straight behind the steps (no host round trip in
-    // between); the launches' error flags are read after it and take
-    // precedence over the walk's status
-    elp_status st = elp_fetch_rings(c->d_lat, c->d_rec, c->g.L, c->N, c->P, c->linear, &c->wb, start, bonds, c->stream);
-    elp_status fl = elp_device_errors(error_flags(c), c->stream);
-    return fl ? fl : st;
+    // the rebuild is queued straight behind the steps (no host round trip in
+    // between); the launches' error flags come back with it and take
+    // precedence over the chains' status
+    return elp_fetch_rings(c->d_lat, c->d_rec, c->g.L, c->N, c->P, c->linear, error_flags(c), &c->wb, start, bonds,
+                           c->stream);
 }
 
 extern "C" elp_status elp_fetch_checked(elp_ctx* c, int32_t* start, uint8_t* bonds, int32_t* code)
@@ -275,10 +274,8 @@ extern "C" elp_status elp_fetch_checked(elp_ctx* c, int32_t* start, uint8_t* bon
     if (!c || !start || !bonds || !code) return elp_fail(ELP_ERR_ARG, "null argument");
     if (!c->loaded) return elp_fail(ELP_ERR_STATE, "no configuration loaded");
     ELP_CUDA_TRY(cudaSetDevice(c->device));
-    elp_status st = elp_fetch_checked_melt(c->d_lat, c->d_rec, c->g.L, c->N, c->P, c->linear, &c->wb, start, bonds,
-                                           code, c->stream);
-    elp_status fl = elp_device_errors(error_flags(c), c->stream);
-    return fl ? fl : st;
+    return elp_fetch_checked_melt(c->d_lat, c->d_rec, c->g.L, c->N, c->P, c->linear, error_flags(c), &c->wb, start,
+                                  bonds, code, c->stream);
 }
 
 extern "C" elp_status elp_observe(elp_ctx* c, double* cms_tuv, double* rg2, double* sl, uint64_t* run_hist,
@@ -287,10 +284,8 @@ extern "C" elp_status elp_observe(elp_ctx* c, double* cms_tuv, double* rg2, doub
     if (!c) return elp_fail(ELP_ERR_ARG, "null argument");
     if (!c->loaded) return elp_fail(ELP_ERR_STATE, "no configuration loaded");
     ELP_CUDA_TRY(cudaSetDevice(c->device));
-    elp_status st = elp_device_errors(error_flags(c), c->stream);
-    if (st) return st;
-    return elp_observe_melt(c->d_lat, c->d_rec, c->g.L, c->N, c->P, c->linear, &c->wb, cms_tuv, rg2, sl, run_hist, nbins,
-                            c->stream);
+    return elp_observe_melt(c->d_lat, c->d_rec, c->g.L, c->N, c->P, c->linear, error_flags(c), &c->wb, cms_tuv, rg2, sl,
+                            run_hist, nbins, c->stream);
 }
 
 extern "C" elp_status elp_check(elp_ctx* c, int32_t* code)
@@ -298,9 +293,7 @@ extern "C" elp_status elp_check(elp_ctx* c, int32_t* code)
     if (!c || !code) return elp_fail(ELP_ERR_ARG, "null argument");
     if (!c->loaded) return elp_fail(ELP_ERR_STATE, "no configuration loaded");
     ELP_CUDA_TRY(cudaSetDevice(c->device));
-    elp_status st = elp_device_errors(error_flags(c), c->stream);
-    if (st) return st;
-    return elp_check_melt(c->d_lat, c->d_rec, c->g.L, c->N, c->P, c->linear, &c->wb, code, c->stream);
+    return elp_check_melt(c->d_lat, c->d_rec, c->g.L, c->N, c->P, c->linear, error_flags(c), &c->wb, code, c->stream);
 }
 
 extern "C" elp_status elp_get_info(const elp_ctx* c, elp_info* info)

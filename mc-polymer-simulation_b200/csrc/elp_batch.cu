@@ -304,8 +304,8 @@ extern "C" elp_status elp_batch_fetch_chains(elp_batch* b, int32_t j, int32_t* s
     if (!start || !bonds) return elp_fail(ELP_ERR_ARG, "null argument");
     const Member& mm = b->m[(size_t)j];
     ELP_CUDA_TRY(cudaSetDevice(b->device));
-    if ((st = errors_of(b, mm.group))) return st;
-    return elp_fetch_rings(mm.lat, mm.rec, mm.g.L, mm.N, mm.P, mm.linear, &b->wb, start, bonds, b->streams[(size_t)mm.group]);
+    return elp_fetch_rings(mm.lat, mm.rec, mm.g.L, mm.N, mm.P, mm.linear, b->d_err + 4 * (size_t)mm.group, &b->wb, start,
+                           bonds, b->streams[(size_t)mm.group]);
 }
 
 extern "C" elp_status elp_batch_observe(elp_batch* b, int32_t j, double* cms_tuv, double* rg2, double* sl,
@@ -315,9 +315,8 @@ extern "C" elp_status elp_batch_observe(elp_batch* b, int32_t j, double* cms_tuv
     if (st) return st;
     const Member& mm = b->m[(size_t)j];
     ELP_CUDA_TRY(cudaSetDevice(b->device));
-    if ((st = errors_of(b, mm.group))) return st;
-    return elp_observe_melt(mm.lat, mm.rec, mm.g.L, mm.N, mm.P, mm.linear, &b->wb, cms_tuv, rg2, sl, run_hist, nbins,
-                            b->streams[(size_t)mm.group]);
+    return elp_observe_melt(mm.lat, mm.rec, mm.g.L, mm.N, mm.P, mm.linear, b->d_err + 4 * (size_t)mm.group, &b->wb, cms_tuv,
+                            rg2, sl, run_hist, nbins, b->streams[(size_t)mm.group]);
 }
 
 extern "C" elp_status elp_batch_get_state(elp_batch* b, int32_t j, uint32_t* words, uint32_t* records)
@@ -340,8 +339,8 @@ extern "C" elp_status elp_batch_check(elp_batch* b, int32_t j, int32_t* code)
     if (!code) return elp_fail(ELP_ERR_ARG, "null argument");
     const Member& mm = b->m[(size_t)j];
     ELP_CUDA_TRY(cudaSetDevice(b->device));
-    if ((st = errors_of(b, mm.group))) return st;
-    return elp_check_melt(mm.lat, mm.rec, mm.g.L, mm.N, mm.P, mm.linear, &b->wb, code, b->streams[(size_t)mm.group]);
+    return elp_check_melt(mm.lat, mm.rec, mm.g.L, mm.N, mm.P, mm.linear, b->d_err + 4 * (size_t)mm.group, &b->wb, code,
+                          b->streams[(size_t)mm.group]);
 }
 
 extern "C" elp_status elp_batch_accepted(elp_batch* b, int32_t j, uint64_t* acc)

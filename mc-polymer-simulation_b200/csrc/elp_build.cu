@@ -156,11 +156,11 @@ elp_status elp_build_melt(uint32_t* lat, uint32_t* rec, int L, int N, int P, int
     elp_status st = elp_walk_bufs_reserve(wb, P, N, 0);
     if (st) return st;
     const size_t S = (size_t)L * L * L;
-    ELP_CUDA_TRY(cudaMemcpyAsync(wb->d_start, start, (size_t)P * 3 * sizeof(int32_t), cudaMemcpyHostToDevice, s));
-    ELP_CUDA_TRY(cudaMemcpyAsync(wb->d_bonds, bonds, (size_t)P * N, cudaMemcpyHostToDevice, s));
+    ELP_CUDA_TRY(cudaMemcpyAsync(wb->d_start(), start, (size_t)P * 3 * sizeof(int32_t), cudaMemcpyHostToDevice, s));
+    ELP_CUDA_TRY(cudaMemcpyAsync(wb->d_bonds(), bonds, (size_t)P * N, cudaMemcpyHostToDevice, s));
     ELP_CUDA_TRY(cudaMemsetAsync(lat, 0, S * sizeof(uint32_t), s));
     elp::BuildArgs a;
-    a.start = wb->d_start; a.bonds = wb->d_bonds; a.lat = lat; a.rec = rec; a.status = wb->d_status;
+    a.start = wb->d_start(); a.bonds = wb->d_bonds(); a.lat = lat; a.rec = rec; a.status = wb->d_status;
     a.L = L; a.N = N; a.P = P; a.linear = linear;
     elp::build_kernel<<<(unsigned)(((size_t)P * 32 + 127) / 128), 128, 0, s>>>(a);
     ELP_CUDA_TRY(cudaGetLastError());

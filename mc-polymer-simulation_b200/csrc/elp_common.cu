@@ -4,6 +4,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -128,6 +129,11 @@ elp_status elp_device_errors(const uint32_t* d_flags, cudaStream_t s)
     uint32_t flags = 0;
     ELP_CUDA_TRY(cudaMemcpyAsync(&flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost, s));
     ELP_CUDA_TRY(cudaStreamSynchronize(s));
+    return elp_flags_status(flags);
+}
+
+elp_status elp_flags_status(uint32_t flags)
+{
     if (flags & 1u)
         return elp_fail(ELP_ERR_STATE, "a domain held more monomer-0 runs than its label table; steps after the "
                                        "overflow are incomplete (use the generic kernel for this melt)");
@@ -139,37 +145,47 @@ elp_status elp_device_errors(const uint32_t* d_flags, cudaStream_t s)
 
 void elp_walk_bufs_free(elp_walk_bufs* b)
 {
-    cudaFree(b->d_start); cudaFree(b->d_bonds); cudaFree(b->d_status); cudaFree(b->d_visit); cudaFree(b->d_cnt);
-    cudaFree(b->d_obs); cudaFree(b->d_rank); cudaFree(b->d_total);
-    cudaFreeHost(b->h_status); cudaFreeHost(b->h_cnt);
+    cudaFree(b->d_out); cudaFree(b->d_status); cudaFree(b->d_visit); cudaFree(b->d_cnt);
+    cudaFree(b->d_obs); cudaFree(b->d_rank);
+    cudaFreeHost(b->h_status); cudaFreeHost(b->h_cnt); cudaFreeHost(b->h_out);
     *b = elp_walk_bufs();
 }
 
 elp_status elp_walk_bufs_reserve(elp_walk_bufs* b, int P, int N, size_t sites)
 {
-    if ((size_t)P > b->cap_rings) {
-        cudaFree(b->d_start); cudaFree(b->d_status);
-        b->d_start = nullptr; b->d_status = nullptr;
-        ELP_CUDA_TRY(cudaMalloc((void**)&b->d_start, (size_t)P * 3 * sizeof(int32_t)));
-        ELP_CUDA_TRY(cudaMalloc((void**)&b->d_status, (size_t)P * sizeof(int32_t)));
-        b->bytes += (size_t)P * 16 - b->cap_rings * 16;
-        b->cap_rings = (size_t)P;
+    b->P = P;
+    b->N = N;
+    if (b->out_bytes() > b->cap_out) {
+        // grow by half at least: a batch's members come in any order of size,
+        // and every growth synchronises the device
+        const size_t need = std::max(b->out_bytes(), b->cap_out + b->cap_out / 2);
+        cudaFree(b->d_out);
+        b->d_out = nullptr;
+        b->bytes -= b->cap_out;
+        b->cap_out = 0;
+        ELP_CUDA_TRY(cudaMalloc((void**)&b->d_out, need));
+        b->cap_out = need;
+        b->bytes += need;
     }
-    if ((size_t)P * N > b->cap_bonds) {
-        cudaFree(b->d_bonds);
-        b->d_bonds = nullptr;
-        ELP_CUDA_TRY(cudaMalloc((void**)&b->d_bonds, (size_t)P * N));
-        b->bytes += (size_t)P * N - b->cap_bonds;
-        b->cap_bonds = (size_t)P * N;
+    if ((size_t)P > b->cap_rings) {
+        cudaFree(b->d_status);
+        b->d_status = nullptr;
+        b->bytes -= b->cap_rings * 4;
+        b->cap_rings = 0;
+        ELP_CUDA_TRY(cudaMalloc((void**)&b->d_status, (size_t)P * sizeof(int32_t)));
+        b->cap_rings = (size_t)P;
+        b->bytes += (size_t)P * 4;
     }
     if (sites > b->cap_sites) {
         cudaFree(b->d_visit);
         b->d_visit = nullptr;
+        b->bytes -= b->cap_sites * 4;
+        b->cap_sites = 0;
         ELP_CUDA_TRY(cudaMalloc((void**)&b->d_visit, sites * sizeof(uint32_t)));
-        b->bytes += (sites - b->cap_sites) * 4;
         b->cap_sites = sites;
+        b->bytes += sites * 4;
     }
-    if (!b->d_cnt) ELP_CUDA_TRY(cudaMalloc((void**)&b->d_cnt, 8 * sizeof(unsigned long long)));
+    if (sites && !b->d_cnt) ELP_CUDA_TRY(cudaMalloc((void**)&b->d_cnt, 8 * sizeof(unsigned long long)));
     return ELP_OK;
 }
 
@@ -186,54 +202,146 @@ static elp_status reserve_host_status(elp_walk_bufs* b, int P)
     return ELP_OK;
 }
 
-elp_status elp_fetch_rings(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear, elp_walk_bufs* b,
-                           int32_t* start, uint8_t* bonds, cudaStream_t s)
+static elp_status reserve_host_out(elp_walk_bufs* b, size_t need)
+{
+    if (need > b->cap_h_out) {
+        if (b->cap_h_out) need = std::max(need, 2 * b->cap_h_out);
+        cudaFreeHost(b->h_out);
+        b->h_out = nullptr;
+        b->cap_h_out = 0;
+        ELP_CUDA_TRY(cudaMallocHost((void**)&b->h_out, need));
+        b->cap_h_out = need;
+    }
+    return ELP_OK;
+}
+
+// Host memory the driver does not know: copies into it are staged.
+static bool pageable(const void* p)
+{
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+// Chains of up to this many bytes go to pageable host buffers through one
+// copy into pinned memory.  One 315 KB copy and a memcpy take 30 us where
+// three staged copies took 60 (L = 64); above it the memcpy costs more than
+// the driver's own staging.
+constexpr size_t STAGE_BYTES = (size_t)1 << 19;
+
+// Wait for the chains queued on the stream and bring them to the host, with
+// the head.
+static elp_status copy_chains(elp_walk_bufs* b, int32_t* start, uint8_t* bonds, elp_chain_head* head, cudaStream_t s)
+{
+    const size_t nb = (size_t)b->P * b->N, ns = (size_t)b->P * 12;
+    const bool far = pageable(start) || pageable(bonds), stage = far && b->out_bytes() <= STAGE_BYTES;
+    elp_status st = reserve_host_out(b, stage ? b->out_bytes() : sizeof(*head));
+    if (st) return st;
+    if (stage) {
+        ELP_CUDA_TRY(cudaMemcpyAsync(b->h_out, b->d_out, b->out_bytes(), cudaMemcpyDeviceToHost, s));
+        ELP_CUDA_TRY(cudaStreamSynchronize(s));
+        memcpy(bonds, b->h_out + (b->d_bonds() - b->d_out), nb);
+        memcpy(start, b->h_out + ((uint8_t*)b->d_start() - b->d_out), ns);
+    } else {
+        ELP_CUDA_TRY(cudaMemcpyAsync(b->h_out, b->d_out, sizeof(*head), cudaMemcpyDeviceToHost, s));
+        if (far) {
+            // fault the buffers' pages in while the device works (a fresh
+            // 2.5 MB buffer took 0.3 ms of the copy behind it)
+            for (size_t i = 0; i < nb; i += 4096) const_cast<volatile uint8_t*>(bonds)[i] = 0;
+            for (size_t i = 0; i < ns; i += 4096) reinterpret_cast<volatile uint8_t*>(start)[i] = 0;
+        }
+        ELP_CUDA_TRY(cudaMemcpyAsync(start, b->d_start(), ns, cudaMemcpyDeviceToHost, s));
+        ELP_CUDA_TRY(cudaMemcpyAsync(bonds, b->d_bonds(), nb, cudaMemcpyDeviceToHost, s));
+        ELP_CUDA_TRY(cudaStreamSynchronize(s));
+    }
+    memcpy(head, b->h_out, sizeof(*head));
+    return ELP_OK;
+}
+
+elp_status elp_fetch_rings(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear,
+                           const uint32_t* flags, elp_walk_bufs* b, int32_t* start, uint8_t* bonds, cudaStream_t s)
 {
     elp_status st = elp_walk_bufs_reserve(b, P, N, 0);
-    if (st || (st = reserve_host_status(b, P))) return st;
-    // list ranking: every run at once, ceil(log2 N) rounds; the chain walk
-    // (one ring's latency) for boxes too large for its scratch
-    const cudaError_t re = elp_rank_chains(lat, rec, L, N, P, linear, b, s);
-    if (re == cudaErrorNotSupported) {
-        WalkArgs w;
-        memset(&w, 0, sizeof(w));
-        w.lat = lat; w.rec = rec; w.L = L; w.N = N; w.P = P; w.linear = linear;
-        w.start = b->d_start; w.bonds = b->d_bonds; w.status = b->d_status;
-        ELP_CUDA_TRY(elp_launch_walk(&w, s));
-    } else {
+    if (st) return st;
+    // list ranking: every chain's segments at once; the chain walk (one
+    // ring's latency) for boxes too large for its scratch
+    const cudaError_t re = elp_rank_chains(lat, rec, L, N, P, linear, true, flags, b, s);
+    if (re != cudaErrorNotSupported) {
         ELP_CUDA_TRY(re);
+        elp_chain_head h;
+        if ((st = copy_chains(b, start, bonds, &h, s))) return st;
+        if ((st = elp_flags_status(h.flags))) return st;
+        if (h.bad || h.chain_monomers != h.site_monomers) {
+            ELP_CUDA_TRY(elp_rank_joined(lat, rec, L, N, P, linear, b, s));
+            ELP_CUDA_TRY(cudaMemcpyAsync(&h, b->d_out, sizeof(h), cudaMemcpyDeviceToHost, s));
+            ELP_CUDA_TRY(cudaStreamSynchronize(s));
+            if (h.bad) return elp_fail(ELP_ERR_INTEGRITY, "chain %d is broken (code 4)", P - (int)h.bad);
+        }
+        return ELP_OK;
     }
-    ELP_CUDA_TRY(cudaMemcpyAsync(start, b->d_start, (size_t)P * 3 * 4, cudaMemcpyDeviceToHost, s));
-    ELP_CUDA_TRY(cudaMemcpyAsync(bonds, b->d_bonds, (size_t)P * N, cudaMemcpyDeviceToHost, s));
+    if ((st = reserve_host_status(b, P))) return st;
+    WalkArgs w;
+    memset(&w, 0, sizeof(w));
+    w.lat = lat; w.rec = rec; w.L = L; w.N = N; w.P = P; w.linear = linear;
+    w.start = b->d_start(); w.bonds = b->d_bonds(); w.status = b->d_status;
+    ELP_CUDA_TRY(elp_launch_walk(&w, s));
+    ELP_CUDA_TRY(cudaMemcpyAsync(start, b->d_start(), (size_t)P * 3 * 4, cudaMemcpyDeviceToHost, s));
+    ELP_CUDA_TRY(cudaMemcpyAsync(bonds, b->d_bonds(), (size_t)P * N, cudaMemcpyDeviceToHost, s));
     ELP_CUDA_TRY(cudaMemcpyAsync(b->h_status, b->d_status, (size_t)P * 4, cudaMemcpyDeviceToHost, s));
     ELP_CUDA_TRY(cudaStreamSynchronize(s));
+    if (flags && (st = elp_device_errors(flags, s))) return st;
     for (int p = 0; p < P; p++)
         if (b->h_status[p])
             return elp_fail(ELP_ERR_INTEGRITY, "chain %d is broken (code %d)", p, b->h_status[p]);
     return ELP_OK;
 }
 
-elp_status elp_fetch_checked_melt(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear,
-                                  elp_walk_bufs* b, int32_t* start, uint8_t* bonds, int32_t* code, cudaStream_t s)
+// The ranked chains hold every monomer of the melt and every site word is in
+// order: integrity code 0.
+static bool all_good(const elp_chain_head& h, int N, int P)
 {
-    const size_t S = (size_t)L * L * L;
-    elp_status st = elp_walk_bufs_reserve(b, P, N, S);
+    return !h.bad && !h.bad_words && h.chain_monomers == h.site_monomers && h.monomers == (unsigned long long)N * P;
+}
+
+elp_status elp_fetch_checked_melt(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear,
+                                  const uint32_t* flags, elp_walk_bufs* b, int32_t* start, uint8_t* bonds,
+                                  int32_t* code, cudaStream_t s)
+{
+    elp_status st = elp_walk_bufs_reserve(b, P, N, 0);
     if (st) return st;
-    if ((st = reserve_host_status(b, P))) return st;
+    const cudaError_t re = elp_rank_chains(lat, rec, L, N, P, linear, true, flags, b, s);
+    if (re != cudaErrorNotSupported) {
+        ELP_CUDA_TRY(re);
+        elp_chain_head h;
+        if ((st = copy_chains(b, start, bonds, &h, s))) return st;
+        if ((st = elp_flags_status(h.flags))) return st;
+        if (all_good(h, N, P)) {
+            *code = 0;
+            return ELP_OK;
+        }
+    }
+    // something is wrong (or the box too large to rank): the walk and the
+    // site scan with visit counters tell efpol's codes apart
+    const size_t S = (size_t)L * L * L;
+    if ((st = elp_walk_bufs_reserve(b, P, N, S)) || (st = reserve_host_status(b, P))) return st;
     if (!b->h_cnt) ELP_CUDA_TRY(cudaMallocHost((void**)&b->h_cnt, 8 * sizeof(unsigned long long)));
     ELP_CUDA_TRY(cudaMemsetAsync(b->d_visit, 0, S * sizeof(uint32_t), s));
     ELP_CUDA_TRY(cudaMemsetAsync(b->d_cnt, 0, 8 * sizeof(unsigned long long), s));
     WalkArgs w;
     memset(&w, 0, sizeof(w));
     w.lat = lat; w.rec = rec; w.L = L; w.N = N; w.P = P; w.linear = linear;
-    w.start = b->d_start; w.bonds = b->d_bonds; w.status = b->d_status; w.visit = b->d_visit; w.counters = b->d_cnt;
+    w.start = b->d_start(); w.bonds = b->d_bonds(); w.status = b->d_status; w.visit = b->d_visit; w.counters = b->d_cnt;
     ELP_CUDA_TRY(elp_launch_walk(&w, s));
     ELP_CUDA_TRY(elp_launch_scan(&w, s));
-    ELP_CUDA_TRY(cudaMemcpyAsync(start, b->d_start, (size_t)P * 3 * 4, cudaMemcpyDeviceToHost, s));
-    ELP_CUDA_TRY(cudaMemcpyAsync(bonds, b->d_bonds, (size_t)P * N, cudaMemcpyDeviceToHost, s));
+    ELP_CUDA_TRY(cudaMemcpyAsync(start, b->d_start(), (size_t)P * 3 * 4, cudaMemcpyDeviceToHost, s));
+    ELP_CUDA_TRY(cudaMemcpyAsync(bonds, b->d_bonds(), (size_t)P * N, cudaMemcpyDeviceToHost, s));
     ELP_CUDA_TRY(cudaMemcpyAsync(b->h_status, b->d_status, (size_t)P * 4, cudaMemcpyDeviceToHost, s));
     ELP_CUDA_TRY(cudaMemcpyAsync(b->h_cnt, b->d_cnt, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     ELP_CUDA_TRY(cudaStreamSynchronize(s));
+    if (flags && (st = elp_device_errors(flags, s))) return st;
     int rc = 0;
     for (int p = 0; p < P && !rc; p++)
         if (b->h_status[p]) rc = 4;
@@ -244,12 +352,28 @@ elp_status elp_fetch_checked_melt(const uint32_t* lat, const uint32_t* rec, int 
     return ELP_OK;
 }
 
-elp_status elp_check_melt(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear, elp_walk_bufs* b,
-                          int32_t* code, cudaStream_t s)
+elp_status elp_check_melt(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear,
+                          const uint32_t* flags, elp_walk_bufs* b, int32_t* code, cudaStream_t s)
 {
-    size_t S = (size_t)L * L * L;
-    elp_status st = elp_walk_bufs_reserve(b, P, N, S);
+    const size_t S = (size_t)L * L * L;
+    elp_status st = elp_walk_bufs_reserve(b, P, N, 0);
     if (st) return st;
+    const cudaError_t re = elp_rank_chains(lat, rec, L, N, P, linear, false, flags, b, s);
+    if (re != cudaErrorNotSupported) {
+        ELP_CUDA_TRY(re);
+        if ((st = reserve_host_out(b, sizeof(elp_chain_head)))) return st;
+        ELP_CUDA_TRY(cudaMemcpyAsync(b->h_out, b->d_out, sizeof(elp_chain_head), cudaMemcpyDeviceToHost, s));
+        ELP_CUDA_TRY(cudaStreamSynchronize(s));
+        elp_chain_head h;
+        memcpy(&h, b->h_out, sizeof(h));
+        if ((st = elp_flags_status(h.flags))) return st;
+        if (all_good(h, N, P)) {
+            *code = 0;
+            return ELP_OK;
+        }
+    }
+    // as elp_fetch_checked_melt
+    if ((st = elp_walk_bufs_reserve(b, P, N, S))) return st;
     ELP_CUDA_TRY(cudaMemsetAsync(b->d_visit, 0, S * sizeof(uint32_t), s));
     ELP_CUDA_TRY(cudaMemsetAsync(b->d_cnt, 0, 8 * sizeof(unsigned long long), s));
     WalkArgs w;
@@ -263,6 +387,7 @@ elp_status elp_check_melt(const uint32_t* lat, const uint32_t* rec, int L, int N
     ELP_CUDA_TRY(cudaMemcpyAsync(status.data(), b->d_status, (size_t)P * 4, cudaMemcpyDeviceToHost, s));
     ELP_CUDA_TRY(cudaMemcpyAsync(cnt, b->d_cnt, sizeof(cnt), cudaMemcpyDeviceToHost, s));
     ELP_CUDA_TRY(cudaStreamSynchronize(s));
+    if (flags && (st = elp_device_errors(flags, s))) return st;
     int rc = 0;
     for (int p = 0; p < P && !rc; p++)
         if (status[(size_t)p]) rc = 4;

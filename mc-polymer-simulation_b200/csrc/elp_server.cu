@@ -231,7 +231,7 @@ static void io_worker(elp_server* s)
         const int lin = j->spec.linear ? 1 : 0;
         int32_t code = -1;
         if (rc == ELP_OK)
-            rc = elp_fetch_checked_melt(sn.d_lat, sn.d_rec, L, N, P, lin, &wb, h_start, h_bonds, &code, st);
+            rc = elp_fetch_checked_melt(sn.d_lat, sn.d_rec, L, N, P, lin, nullptr, &wb, h_start, h_bonds, &code, st);
         std::string err = rc == ELP_OK ? std::string() : std::string(elp_last_error());
         cudaFreeAsync(sn.d_lat, st);
         cudaFreeAsync(sn.d_rec, st);
