@@ -137,10 +137,14 @@ struct Shape {
     // with the next group's after its first barrier
     static constexpr bool fits(int words) { return (size_t)MINB * ((size_t)words * 4 + 1024) <= 233472; }
     static constexpr bool PRE = !PER && fits(RNDW + NG * A);
-    // where it fits too: a second table with each entry's change of the
-    // anchor's word (four instructions of a substep's 48)
+    // Small whole boxes, bound by latency: a second table with each entry's
+    // change of the anchor's word takes four instructions out of the move
+    // (L = 16: 10.6 -> 10.4 us per step, L = 24: 20.2 -> 19.3).  Its loads'
+    // bank conflicts cost more where the SM is full (L = 32: 29.5 against
+    // 30.4, L = 128: 18.2 against 18.4, 48x24x24 tiles at L = 192: 62.8
+    // against 66.3).
     static constexpr int DTABW = RNDW + (PRE ? NG : 1) * A;
-    static constexpr bool DT = fits(DTABW + ELP_MOVE_ENTRIES);
+    static constexpr bool DT = PER && K == 1;
     static constexpr int TOTW = DTABW + (DT ? ELP_MOVE_ENTRIES : 0);
     static constexpr size_t BYTES = (size_t)TOTW * 4;
     // neighbour offsets in words fit 16 signed bits (else they are taken
