@@ -293,40 +293,57 @@ __device__ __forceinline__ Span grid_span()
 {
     return Span{blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x};
 }
-__global__ void __launch_bounds__(256) rank_segments(RankArgs a)
+// Zero the head and the bonds (`clear` bytes) for the kernels behind.
+__device__ __forceinline__ void clear_out(const RankArgs& a, Span sp, size_t clear)
 {
+    uint4* zero = reinterpret_cast<uint4*>(a.head);
+    for (size_t i = sp.first; i < clear / 16; i += sp.count) zero[i] = make_uint4(0, 0, 0, 0);
+}
+__device__ __forceinline__ void all_chain_checks(const RankArgs& a, Span sp, int fin)
+{
+    chain_checks(a, sp, fin);
+    if (sp.first == 0 && a.flags) a.head->flags = *a.flags;
+}
+__global__ void __launch_bounds__(256) rank_segments(RankArgs a, size_t clear)
+{
+    clear_out(a, grid_span(), clear);
     segments(a, grid_span());
-    scan_words(a, grid_span());
 }
 __global__ void __launch_bounds__(256) rank_round(RankArgs a, int r) { round_of(a, grid_span(), r); }
-__global__ void __launch_bounds__(256) rank_chains(RankArgs a, int fin)
+__global__ void __launch_bounds__(256) rank_chains(RankArgs a, int fin) { all_chain_checks(a, grid_span(), fin); }
+__global__ void __launch_bounds__(256) rank_bonds(RankArgs a, int fin)
 {
-    chain_checks(a, grid_span(), fin);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && a.flags) a.head->flags = *a.flags;
+    write_bonds(a, grid_span(), fin);
+    scan_words(a, grid_span());
 }
-__global__ void __launch_bounds__(256) rank_bonds(RankArgs a, int fin) { write_bonds(a, grid_span(), fin); }
 
-// Small boxes: the same in one launch of one cluster.  The phases hand their
-// results over through global memory: each ends in a cluster barrier, which
-// releases and acquires them, and loads that cross it bypass L1.
-__global__ void __launch_bounds__(1024) rank_cluster(RankArgs a, int rounds, size_t clear)
+// Phases in one launch of one cluster: they hand their results over through
+// global memory, and each ends in a cluster barrier, which releases and
+// acquires them; loads that cross it bypass L1.
+__device__ __forceinline__ void cluster_rounds(const RankArgs& a, Span sp, cg::cluster_group& cl, int rounds)
 {
-    cg::cluster_group cl = cg::this_cluster();
-    const Span sp = grid_span();
-    uint32_t* zero = reinterpret_cast<uint32_t*>(a.head);
-    for (size_t i = sp.first; i < clear / 4; i += sp.count) zero[i] = 0u;
-    segments(a, sp);
-    cl.sync();
-    scan_words(a, sp);
     for (int r = 0; r < rounds; r++) {
         round_of(a, sp, r);
         cl.sync();
     }
-    const int fin = rounds & 1;
-    chain_checks(a, sp, fin);
-    if (sp.first == 0 && a.flags) a.head->flags = *a.flags;
+    all_chain_checks(a, sp, rounds & 1);
+}
+__global__ void __launch_bounds__(1024) rank_cluster(RankArgs a, int rounds, size_t clear)
+{
+    cg::cluster_group cl = cg::this_cluster();
+    const Span sp = grid_span();
+    clear_out(a, sp, clear);
+    segments(a, sp);
     cl.sync();
-    write_bonds(a, sp, fin);
+    cluster_rounds(a, sp, cl, rounds);
+    cl.sync();
+    write_bonds(a, sp, rounds & 1);
+    scan_words(a, sp);
+}
+__global__ void __launch_bounds__(1024) rank_cluster_rounds(RankArgs a, int rounds)
+{
+    cg::cluster_group cl = cg::this_cluster();
+    cluster_rounds(a, grid_span(), cl, rounds);
 }
 
 // Only when the sums disagree: monomers of all runs that reach each chain's
@@ -383,7 +400,9 @@ cudaError_t grow(void** p, size_t* cap, size_t need, size_t* bytes)
 // Boxes up to this many sites (40^3) are ranked by one cluster, whose barriers
 // replace a dozen launches: a fetch at L = 32 takes 68 us, 95 by launches.
 // At L = 64 eight SMs are too few: 194 us by the cluster, 105 by launches.
-constexpr size_t CLUSTER_SITES = (size_t)1 << 16;
+// Up to CLUSTER_NODES nodes (some 56^3 sites) they still do the rounds: L = 48
+// 78 us, 88 by launches (L = 64: 113 and 105).
+constexpr size_t CLUSTER_SITES = (size_t)1 << 16, CLUSTER_NODES = 3 << 14;
 constexpr int CLUSTER = 8;   // CTAs (portable cluster size)
 
 RankArgs rank_args(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear, elp_walk_bufs* b)
@@ -430,7 +449,9 @@ cudaError_t elp_rank_chains(const uint32_t* lat, const uint32_t* rec, int L, int
     int R = 0;
     while ((1L << R) < (long)N) R++;
     const size_t clear = want_bonds ? b->clear_bytes() : sizeof(elp_chain_head);
-    if (S <= CLUSTER_SITES) {
+    const int blocks = (int)((nodes + 255) / 256 < 148 * 8 ? (nodes + 255) / 256 : 148 * 8), fin = R & 1;
+    if (S > CLUSTER_SITES) rank_segments<<<blocks, 256, 0, s>>>(a, clear);
+    if (nodes <= CLUSTER_NODES) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(CLUSTER);
         cfg.blockDim = dim3(1024);
@@ -441,13 +462,12 @@ cudaError_t elp_rank_chains(const uint32_t* lat, const uint32_t* rec, int L, int
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, rank_cluster, a, R, clear);
+        if (S <= CLUSTER_SITES) return cudaLaunchKernelEx(&cfg, rank_cluster, a, R, clear);
+        if ((e = cudaLaunchKernelEx(&cfg, rank_cluster_rounds, a, R)) != cudaSuccess) return e;
+    } else {
+        for (int r = 0; r < R; r++) rank_round<<<blocks, 256, 0, s>>>(a, r);
+        rank_chains<<<(P + 255) / 256, 256, 0, s>>>(a, fin);
     }
-    if ((e = cudaMemsetAsync(a.head, 0, clear, s)) != cudaSuccess) return e;
-    const int blocks = (int)((nodes + 255) / 256 < 148 * 8 ? (nodes + 255) / 256 : 148 * 8), fin = R & 1;
-    rank_segments<<<blocks, 256, 0, s>>>(a);
-    for (int r = 0; r < R; r++) rank_round<<<blocks, 256, 0, s>>>(a, r);
-    rank_chains<<<(P + 255) / 256, 256, 0, s>>>(a, fin);
     rank_bonds<<<blocks, 256, 0, s>>>(a, fin);
     return cudaGetLastError();
 }
