@@ -89,6 +89,7 @@ struct Shape {
     static constexpr int A = R * (TX / NC);   // anchors per substep
     static constexpr int G = A / 4;           // Philox counters per substep group
     static constexpr int AT = A / K;          // threads that own anchors
+    static constexpr bool TILED = !PER;
     static constexpr int THREADS = (AT + 31) / 32 * 32;
     static constexpr bool TAIL = AT != THREADS;   // threads without anchors fill the last warp
     // Tiled domains: row y of plane z starts at OX + SX y + SXY z (16-byte
@@ -130,21 +131,25 @@ struct Shape {
     static constexpr int RNDW = (HTABW + 64 + 3) & ~3;
     static constexpr int NSUB = 2 * NC;              // substeps per step
     static constexpr int NG = (NSUB + 3) / 4;        // groups of four substeps
-    // Random bytes, one word (four substeps) per anchor and group: in tiled
-    // domains, where MINB CTAs still fit on an SM (228 KB, 1 KB reserved per
-    // CTA), all NG groups of the step, drawn before its substeps (PRE); else
-    // one group's, read into registers as the group starts and overwritten
-    // with the next group's after its first barrier
+    // Random bytes, one word (four substeps) per anchor and group.  With one
+    // anchor a thread, and where MINB CTAs still fit on an SM (228 KB, 1 KB
+    // reserved per CTA), all NG groups of the step, drawn before its substeps
+    // (PRE): no warp is late at a barrier for drawing (L = 16: 10.4 -> 9.9 us
+    // per step, L = 24: 19.3 -> 18.8).  Else one group's, read into registers
+    // as the group starts and overwritten with the next group's after its
+    // first barrier: with two anchors a thread the SM is full anyway (drawn
+    // ahead, L = 32 took 30.3 against 29.5, 48x24x24 tiles at L = 192 65.5
+    // against 62.8).
     static constexpr bool fits(int words) { return (size_t)MINB * ((size_t)words * 4 + 1024) <= 233472; }
-    static constexpr bool PRE = !PER && fits(RNDW + NG * A);
-    // Small whole boxes, bound by latency: a second table with each entry's
-    // change of the anchor's word takes four instructions out of the move
-    // (L = 16: 10.6 -> 10.4 us per step, L = 24: 20.2 -> 19.3).  Its loads'
-    // bank conflicts cost more where the SM is full (L = 32: 29.5 against
-    // 30.4, L = 128: 18.2 against 18.4, 48x24x24 tiles at L = 192: 62.8
-    // against 66.3).
+    static constexpr bool PRE = K == 1 && fits(RNDW + NG * A);
+    // One CTA of one anchor a thread per SM is bound by latency: a second table
+    // with each entry's change of the anchor's word takes four instructions
+    // out of the move (L = 24: 20.2 -> 19.3 us per step, L = 72: 22.3 -> 21.7).
+    // Its loads' bank conflicts cost more where the SM is full (L = 32: 29.5
+    // against 30.4, L = 128: 18.2 against 18.4, 48x24x24 tiles at L = 192:
+    // 62.8 against 66.3).
     static constexpr int DTABW = RNDW + (PRE ? NG : 1) * A;
-    static constexpr bool DT = PER && K == 1;
+    static constexpr bool DT = K == 1 && MINB == 1 && fits(DTABW + ELP_MOVE_ENTRIES);
     static constexpr int TOTW = DTABW + (DT ? ELP_MOVE_ENTRIES : 0);
     static constexpr size_t BYTES = (size_t)TOTW * 4;
     // neighbour offsets in words fit 16 signed bits (else they are taken
@@ -240,6 +245,22 @@ __device__ __forceinline__ void follow_label(int p, int pB, int pY, uint32_t wP,
     }
 }
 
+// The tile at hand, in shared memory: what its load and store need, which
+// would otherwise hold registers through the substeps.
+struct Tile {
+    uint32_t* lat;
+    uint32_t* rec;
+    uint2 key;
+    uint32_t t;         // absolute step
+    int d, L;           // domain, box edge
+    int x0, y0, z0;     // box site of the tile's first word
+    unsigned long long* acc;
+};
+static_assert(sizeof(Tile) <= 80, "20 words of shared memory");
+// The tile at hand and the next one are slots par and par ^ 1.
+template <class SH>
+__device__ __forceinline__ Tile& tile(int par) { return *reinterpret_cast<Tile*>(g_smem + SH::TILEW + 20 * par); }
+
 // Random bytes of one substep group: byte q of words 0-3 of Philox counter
 // {t, d, group, gq} serves anchor gq + q G in the group's four substeps: bit
 // 0 the slot s, bits 1-4 the table option.  Kept as one word per anchor, a
@@ -299,22 +320,6 @@ __device__ __forceinline__ uint4 draw_schedule(uint32_t t, int d, uint2 key)
     return w;
 }
 
-// The tile at hand, in shared memory: what its load and store need, which
-// would otherwise hold registers through the substeps.
-struct Tile {
-    uint32_t* lat;
-    uint32_t* rec;
-    uint2 key;
-    uint32_t t;         // absolute step
-    int d, L;           // domain, box edge
-    int x0, y0, z0;     // box site of the tile's first word
-    unsigned long long* acc;
-};
-static_assert(sizeof(Tile) <= 80, "20 words of shared memory");
-// The tile at hand and the next one are slots par and par ^ 1.
-template <class SH>
-__device__ __forceinline__ Tile& tile(int par) { return *reinterpret_cast<Tile*>(g_smem + SH::TILEW + 20 * par); }
-
 // Set up a tile (one warp): domain item.y of melt J at `step`.
 template <class SH, int TX, int TY, int TZ, int NC>
 __device__ __forceinline__ void set_tile(const BatchJob& J, int d, uint32_t step, int par)
@@ -348,7 +353,7 @@ __device__ __forceinline__ void fill_slots(const Tile& T, uint32_t ns)
     const uint32_t tid = threadIdx.x;
     uint4 rr = make_uint4(0, 0, 0, 0);
     if (tid < ns) rr = __ldcg(reinterpret_cast<const uint4*>(T.rec + ELP_REC_WORDS * (size_t)g_smem[SH::SCHW + tid]));
-    if (SH::PRE) draw_step<SH, 1>(T.t, T.d, T.key);
+    if (SH::PRE && SH::TILED) draw_step<SH, 1>(T.t, T.d, T.key);
     for (uint32_t sl = tid; sl < ns; sl += SH::THREADS) {
         if (sl != tid) rr = __ldcg(reinterpret_cast<const uint4*>(T.rec + ELP_REC_WORDS * (size_t)g_smem[SH::SCHW + sl]));
         const uint32_t idx = g_smem[SH::SLOW + sl];
@@ -677,7 +682,12 @@ __global__ void __launch_bounds__(((TX * TX * (TX / NC) / K) + 31) / 32 * 32, 1)
         unsigned long long accepted = 0;
         for (int st = 0; st < a.nsteps; st++) {
             const uint32_t t = t0 + (uint32_t)st;
-            if (tid < SH::G) draw_bytes<SH>(random_words<SH>(0), t, 0, 0, tid, key);
+            if (SH::PRE) {
+                draw_step<SH, 0>(t, 0, key);
+                draw_step<SH, 1>(t, 0, key);
+            } else if (tid < SH::G) {
+                draw_bytes<SH>(random_words<SH>(0), t, 0, 0, tid, key);
+            }
             if (tid >= SH::THREADS - 32) draw_schedule<SH, NC>(t, 0, key);
             if (tid == 0) {
                 tile<SH>(0).t = t;
