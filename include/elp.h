@@ -212,15 +212,15 @@ elp_status elp_set_state(elp_ctx* ctx, const uint32_t* words, const uint32_t* re
  * an error (its steps are incomplete), as elp_sync does. */
 elp_status elp_accepted(elp_ctx* ctx, uint64_t* accepted);
 
-/* Bound of the grid-barrier waits inside tiled launches of several steps.
+/* Bound of the waits inside launches of several steps (tiles: at the grid
+ * barrier between steps; a box in slabs: of a slab for its neighbours).
  * No counterpart in the reference, whose launches take one step each
- * (gpupol2/gpupol_cuda.cu:129-146).  Between two steps the CTAs of a launch
- * meet at a grid barrier; a wait gives up after `polls` polls (0: the
- * default, about a second), the launch stops there and reports
+ * (gpupol2/gpupol_cuda.cu:129-146).  A wait gives up after `polls` polls (0:
+ * the default, about a second), the launch stops there and reports
  * ELP_ERR_STATE at the next synchronising call.  The context stays usable:
  * loading a configuration (elp_init_melt, a load call, elp_set_state) clears
  * the report.  hold_block >= 0 is a test hook: that CTA of each later launch
- * never arrives at the first barrier, so every wait there runs out of polls
+ * goes no further than its first step, so every wait for it runs out of polls
  * -- the failure path is tested without faulting or hanging the GPU.  -1
  * lets every CTA arrive. */
 elp_status elp_debug_waits(elp_ctx* ctx, uint32_t polls, int32_t hold_block);

@@ -138,8 +138,8 @@ elp_status elp_flags_status(uint32_t flags)
         return elp_fail(ELP_ERR_STATE, "a domain held more monomer-0 runs than its label table; steps after the "
                                        "overflow are incomplete (use the generic kernel for this melt)");
     if (flags & 4u)
-        return elp_fail(ELP_ERR_STATE, "a tiled launch of several steps gave up waiting at its grid barrier; steps "
-                                       "after it are incomplete");
+        return elp_fail(ELP_ERR_STATE, "a launch of several steps gave up waiting (tiles: at its grid barrier; slabs of "
+                                       "a box: for each other); steps after it are incomplete");
     return ELP_OK;
 }
 

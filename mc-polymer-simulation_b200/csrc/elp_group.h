@@ -22,6 +22,7 @@ struct elp_group {
     int threads;                      // block size of the sweep kernel in use
     size_t smem;                      // its dynamic shared memory per block
     int spl;                          // steps per launch (tiled: specialised kernel only)
+    int alone = 0;                    // set before commit: no other group's work runs beside this one's
     int use_graph;                    // tiled domains: replay launches from a CUDA graph
     int graph_steps;                  // steps captured per graph (rounded down to whole launches)
     cudaStream_t stream;
@@ -36,8 +37,8 @@ struct elp_group {
     size_t cap_jobs = 0, cap_items = 0;   // grow-only device capacity of the two tables
     uint32_t* d_moves = nullptr;      // move table and neighbour offsets (elp_move_table)
     uint32_t* d_ctr = nullptr;        // device step counter, then the grid barrier's two counts
-    uint32_t wait_polls = 0;          // bound of the grid barrier's waits (0: the kernel's default)
-    int hold_cta1 = 0;                // test hook: CTA + 1 that never arrives at the first barrier
+    uint32_t wait_polls = 0;          // bound of the waits inside a launch (0: the kernel's default)
+    int hold_cta1 = 0;                // test hook: CTA + 1 that stops after a launch's first step
     uint64_t steps_done = 0;          // steps since the job table's step0 values
     uint32_t ctr_mirror = 0;          // host copy of *d_ctr
     uint64_t kernels = 0;             // sweep-path kernels launched (graph replays count their nodes)

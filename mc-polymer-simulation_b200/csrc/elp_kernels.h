@@ -52,10 +52,10 @@ struct BatchLaunch {
     const uint32_t* table;         // 4096-byte transition table
     const uint32_t* moves;         // move table and neighbour offsets of the geometry (elp_move_table)
     uint32_t* error;               // device error flags (bit 0: label slot table overflow,
-                                   // bit 2: a grid barrier wait gave up)
+                                   // bit 2: a wait of a launch gave up)
     uint32_t* grid_bar;            // tiled domains, nsteps > 1: {arrivals, exits}, zero between launches
-    uint32_t wait_polls;           // polls before a grid barrier wait gives up (0: about a second)
-    int hold_cta1;                 // test hook: CTA + 1 that never arrives at the first barrier (0: none)
+    uint32_t wait_polls;           // polls before a wait gives up (0: about a second)
+    int hold_cta1;                 // test hook: CTA + 1 that stops after the first step (0: none)
 };
 
 #include "elp_internal.h"
@@ -68,6 +68,7 @@ struct Sweep2Launch {
     BatchLaunch args;
     int threads_out;               // check_only: block size of the kernel that fits
     size_t smem_out;               // check_only: its dynamic shared memory
+    int alone;                     // 1: no other group's work shares the device with this one
     int linear;                    // 1: some job holds linear chains (kernel with monomer-0 moves)
 };
 

@@ -23,7 +23,9 @@
 //     anchors from an 8 x 4 block of rows so that their first loads hit 32
 //     different banks;
 //   * the grid is persistent over the tiles, and a launch of several steps
-//     over a tiled box is cooperative, with a grid barrier between steps.
+//     over a tiled box is cooperative, with a grid barrier between steps;
+//   * whole boxes of rings have kernels of their own (sweep_slabs), in slabs
+//     on the CTAs of a cluster where one SM would be the bound.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -134,8 +136,8 @@ struct Shape {
     // Random bytes, one word (four substeps) per anchor and group.  With one
     // anchor a thread, and where MINB CTAs still fit on an SM (228 KB, 1 KB
     // reserved per CTA), all NG groups of the step, drawn before its substeps
-    // (PRE): no warp is late at a barrier for drawing (L = 16: 10.4 -> 9.9 us
-    // per step, L = 24: 19.3 -> 18.8).  Else one group's, read into registers
+    // (PRE): no warp is late at a barrier for drawing (rings of L = 16 in
+    // sweep_box: 10.4 -> 9.9 us per step, L = 24: 19.3 -> 18.8).  Else one group's, read into registers
     // as the group starts and overwritten with the next group's after its
     // first barrier: with two anchors a thread the SM is full anyway (drawn
     // ahead, L = 32 took 30.3 against 29.5, 48x24x24 tiles at L = 192 65.5
@@ -144,7 +146,8 @@ struct Shape {
     static constexpr bool PRE = K == 1 && fits(RNDW + NG * A);
     // One CTA of one anchor a thread per SM is bound by latency: a second table
     // with each entry's change of the anchor's word takes four instructions
-    // out of the move (L = 24: 20.2 -> 19.3 us per step, L = 72: 22.3 -> 21.7).
+    // out of the move (rings of L = 24 in sweep_box: 20.2 -> 19.3 us per step,
+    // L = 72: 22.3 -> 21.7).
     // Its loads' bank conflicts cost more where the SM is full (L = 32: 29.5
     // against 30.4, L = 128: 18.2 against 18.4, 48x24x24 tiles at L = 192:
     // 62.8 against 66.3).
@@ -637,7 +640,8 @@ __device__ __forceinline__ void load_tables(const BatchLaunch& a)
     for (int i = threadIdx.x; i < 64; i += SH::THREADS) g_smem[SH::HTABW + i] = a.table[960 + i];
 }
 
-// Whole boxes: each CTA holds one melt for all steps of the launch.
+// Whole boxes of linear chains, and of rings where sweep_slabs below does not
+// run: each CTA holds one melt for all steps of the launch.
 //
 // K anchors per thread: K = 2 where a domain has more than 1024 anchors per
 // substep, else 1 (more warps hide latency better than more moves in flight
@@ -703,6 +707,343 @@ __global__ void __launch_bounds__(((TX * TX * (TX / NC) / K) + 31) / 32 * 32, 1)
             lat[i] = wv;
         }
         count_accepted(J.acc, accepted);
+    }
+}
+
+// ---- whole boxes of rings, one anchor a thread -----------------------------------
+//
+// A box of 32^3 on one SM (sweep_box) is bound by that SM's issue slots and
+// shared-memory wavefronts: 2048 anchors a substep, 29.5 us per step.  Here it
+// lies in C slabs of whole planes on the CTAs of a cluster.  Each slab holds a
+// copy of the plane below and of the plane above, so that a move, which
+// touches the anchor's neighbours at most, reads this CTA's shared memory
+// only; a new word that another slab holds too is sent there.  15.9 us per
+// step with C = 8.
+//
+// What it took: words fetched from the neighbouring slab instead of kept as
+// copies 26.5 us; a cluster barrier (release, acquire) per substep 20.9, as it
+// waits for every store to be acknowledged (0.31 us in a loop of its own,
+// against 0.13 for a barrier of arrivals that announce bytes); C = 4: 20.3.
+// L = 30: 28.3 -> 17.6, L = 28: 24.0 -> 14.2.  L = 26 has slabs of 13 planes
+// only: 20.1 -> 23.0, left alone.
+//
+// The boxes that fit the threads of one CTA (up to 24^3) run as one slab: they
+// too are bound by latency, and gain from monomer 0's offsets kept by site
+// (see slab_substep).  L = 16: 9.9 -> 8.95 us per step (N = 50; N = 20: 11.2
+// -> 10.1), L = 18: 12.5 -> 11.5, L = 20: 14.4 -> 13.8, L = 22: 16.6 -> 16.3,
+// L = 24: 18.8 -> 18.6.
+__device__ __forceinline__ uint32_t cluster_address(uint32_t rank)   // of a CTA's g_smem
+{
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(g_smem)), "r"(rank));
+    return a;
+}
+// Barrier over the cluster, in two halves: stores before the arrival, to this
+// CTA's shared memory or another's, are seen after the wait.
+__device__ __forceinline__ void cluster_arrive()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Wait for the completion of a phase of an mbarrier; false when it gave up
+// after `polls` tries of a microsecond at most.
+constexpr uint32_t SLAB_POLLS = 1u << 20;
+__device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity, uint32_t polls)
+{
+    for (uint32_t n = 0; n < polls; n++) {
+        uint32_t done;
+        asm volatile("{\n.reg .pred q;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], %2, 1000;\n"
+                     "selp.u32 %0, 1, 0, q;\n}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+// Slab of ZS planes of a box shared by C CTAs.  C > 1: on chip with a copy of
+// the plane below and of the plane above (planes 0 and ZS + 1).
+template <int TX, int NC, int SX, int SXY, int C>
+struct Slab {
+    static constexpr int ZS = TX / C, R = TX * TX, HALO = C > 1 ? 1 : 0, PLANES = ZS + 2 * HALO;
+    static constexpr int A = R * (TX / NC), G = A / 4;      // anchors and counters of the whole box
+    // one anchor a thread, WP x groups of each row; a warp's lanes take the
+    // rows of one plane if there are other slabs
+    static constexpr int WP = TX / NC, ROWS = C > 1 ? 32 : TX, THREADS = (ROWS * WP * ZS + 31) / 32 * 32;
+    __device__ static bool idle()
+    {
+        return (ROWS != TX && (int)threadIdx.x % ROWS >= TX) || (ROWS * WP * ZS != THREADS && (int)threadIdx.x >= ROWS * WP * ZS);
+    }
+    static constexpr int NSUB = 2 * NC, NG = (NSUB + 3) / 4;
+    // a labelled word holds its chain + 1 above bit LSH; monomer 0's offset
+    // in the run at a site has a word of its own, copied as the site's is
+    static constexpr int LSH = 4;
+    static constexpr uint32_t LMASK = 0xFFF0u;
+    static constexpr int MAXCHAINS = LMASK >> LSH;
+    static constexpr int TABW = (SXY * PLANES + 3) & ~3;
+    static constexpr int OFFW = TABW + ELP_MOVE_ENTRIES;
+    static constexpr int TABS = ELP_MOVE_ENTRIES + 27 * 16;
+    static constexpr int DTABW = TABW + TABS;
+    static constexpr int OFSW = DTABW + ELP_MOVE_ENTRIES;   // offsets by site
+    static constexpr int COLW = OFSW + TABW;                // colours of a step and the next
+    static constexpr int BARW = COLW + 8 * NG;              // two mbarriers
+    static constexpr size_t BYTES = (size_t)(BARW + 4) * 4;
+    static_assert(TX % C == 0 && C <= 8 && THREADS <= 1024 && A % 4 == 0 && TABS % 4 == 0, "slabs of whole planes");
+    static_assert(C == 1 || (TX <= 32 && ZS >= 4), "a warp's anchors lie in one plane and reach one other slab at most");
+    static_assert((TX - 1) * (1 + SX + (C > 1 ? 0 : SXY)) + SXY <= 32767, "neighbour offsets in 16 signed bits");
+    static_assert(BYTES <= 232448, "dynamic shared memory of one CTA");
+};
+
+// The words of anchor gq + q G for one substep group, as draw_bytes keeps them.
+__device__ __forceinline__ uint32_t own_bytes(uint32_t t, int group, uint32_t gq, uint32_t sel, uint2 key)
+{
+    const uint4 v = philox(make_uint4(t, 0u, (uint32_t)group, gq), key);
+    const uint32_t w = __byte_perm(__byte_perm(v.x, v.y, sel), __byte_perm(v.z, v.w, sel), 0x5410);
+    return ((w << 7) & 0x80808080u) | ((w << 1) & 0x3C3C3C3Cu);
+}
+
+// Slabs: where a warp's new words go besides this CTA's copy.  Words of byte
+// offsets from .. from + len - 1 are sent to the slab below or above (cluster
+// address `to` plus the byte offset), announced at that slab's mbarrier.
+struct Push {
+    uint32_t to, bar, len;
+    int from;
+    uint32_t sent;      // bytes this thread has sent in the substep
+};
+// Word at byte offset b, belonging to the site at offset `site`.  Predicated:
+// with branches around the sends L = 32 took 18.7 us per step, so 15.9.
+__device__ __forceinline__ void push_word(Push& o, bool ok, int site, int b, uint32_t w)
+{
+    const uint32_t go = ok && (uint32_t)(site - o.from) < o.len ? 4u : 0u;
+    asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %3, 0;\n"
+                 "@q st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];\n}"
+                 ::"r"(o.to + (uint32_t)b), "r"(w), "r"(o.bar), "r"(go) : "memory");
+    o.sent += go;
+}
+
+// One substep of a slab: the move of substepK, one anchor a thread.  What
+// bounds a slab is the chain of latencies from barrier to barrier (a warp or
+// two per scheduler), so monomer 0's offsets at the runs that it may leave or
+// be joined in are fetched along with the words, the new words are complete
+// before they are stored, and each is sent once (words sent to one address
+// would arrive in any order).
+template <class SH, int NC, int KK>
+__device__ __forceinline__ uint32_t slab_substep(const Anchors<1>& an, uint32_t rw, int c4, Push& push)
+{
+    const int xr4 = colour_x<NC>(c4, an.rot[0]);
+    const int p = an.base[0] + xr4;
+    const int tc = an.cls[0] + (xr4 == an.xlo[0] ? -64 : 0) + (xr4 == an.xhi[0] ? 64 : 0);
+    uint32_t wP = SW(p), R = spread_byte<KK>(rw);
+    if (SH::idle()) wP = R = 0;   // slot 0 of an empty site: no move
+    const uint32_t V = SW(tc + (int)((wP & 15) << 2));
+    const int pB = p + ((int)V >> 14);
+    const bool s = (R & 0x8000u) != 0;
+    const uint32_t w1 = SW(pB), wB = s ? w1 : wP;
+    const int from = s ? pB : p;              // the run that the monomer leaves
+    const uint32_t oB = SW(4 * SH::OFSW + from);
+    const bool c2 = wB >= 2u * ELP_CUNIT;
+    uint32_t ix = R & (V | 0x3Cu);
+    if (c2 != s) ix += (wB & 15) << 6;
+    const uint32_t E = SW(4 * SH::TABW + (int)ix), D = SW(4 * SH::DTABW + (int)ix);
+    const uint32_t V2 = SW(tc + (int)(E >> 26));
+    const int pY = p + ((int)V2 >> 14);
+    const uint32_t wY = SW(pY), oY = SW(4 * SH::OFSW + pY);
+    const bool ok = E != 0 && (wY & E & 0xFu) == 0, away = (E >> 28) != 0;   // away: not into the anchor's run
+    uint32_t nP = wP + D, nB = c2 ? wB - ELP_CUNIT : 0u, nY = wY + ELP_CUNIT + ((E >> 9) & 15u);
+    int at = -1;                              // the run with monomer 0 whose offset changes
+    uint32_t off = 0;
+    if (ok && ((wB | wY) & SH::LMASK)) {
+        const uint32_t lb = wB & SH::LMASK;
+        if (lb) {
+            off = oB;
+            at = from;
+            if (off == (s ? 0u : (wB >> ELP_CSHIFT) - 1)) {   // monomer 0 is the one that moves
+                (s ? nB : nP) &= ~SH::LMASK;
+                (away ? nY : nP) |= lb;
+                off = away ? 0u : (nP >> ELP_CSHIFT) - 1;
+                at = pY;
+            } else if (s) {
+                off--;
+            }
+        } else if (away) {                    // one joins the front of its run
+            off = oY + 1;
+            at = pY;
+        }
+    }
+    if (ok && away) SW(pY) = nY;
+    if (ok && s) SW(pB) = nB;
+    if (ok) SW(p) = nP;
+    if (at >= 0) SW(4 * SH::OFSW + at) = off;
+    if (SH::HALO) {
+        push_word(push, ok && away, pY, pY, nY);
+        push_word(push, ok && s, pB, pB, nB);
+        push_word(push, ok, p, p, nP);
+        push_word(push, at >= 0, at, 4 * SH::OFSW + at, off);
+    }
+    return ok ? 1u : 0u;
+}
+
+template <int TX, int NC, int SX, int SXY, int C>
+__global__ void __launch_bounds__(Slab<TX, NC, SX, SXY, C>::THREADS, 1) sweep_slabs(BatchLaunch a)
+{
+    using SH = Slab<TX, NC, SX, SXY, C>;
+    uint32_t* S = g_smem;
+    const int tid = threadIdx.x;
+    uint32_t rank = 0;
+    if (C > 1) asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int row = tid / SH::ROWS, zl = row % SH::ZS, j = SH::idle() ? 0 : row / SH::ZS;
+    // the two lowest planes' warps write words that the slab below holds too
+    // (its planes ZS and ZS + 1), the two highest planes' the slab above
+    Push push = {};
+    const bool sends = C > 1 && (zl < 2 || zl >= SH::ZS - 2);   // the same for a warp
+    if (sends) {
+        const uint32_t at = cluster_address(zl < 2 ? (rank == 0 ? C - 1 : rank - 1) : (rank + 1 == C ? 0 : rank + 1));
+        push.to = zl < 2 ? at + 4 * SXY * SH::ZS : at - 4 * SXY * SH::ZS;
+        push.bar = at + 4 * SH::BARW;
+        push.from = zl < 2 ? 0 : 4 * SXY * SH::ZS;
+        push.len = 8 * SXY;
+    }
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(S + SH::BARW);
+    if (C > 1 && tid == 0) {
+        // one arrival of each warp that sends here
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(4 * SH::WP) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar + 8), "r"(4 * SH::WP) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int i = tid; i < SH::TABS / 4; i += SH::THREADS) cp_async16(S + SH::TABW + 4 * i, a.moves + 4 * i);
+    for (int i = tid; i < ELP_MOVE_ENTRIES / 4; i += SH::THREADS)
+        cp_async16(S + SH::DTABW + 4 * i, a.moves + SH::TABS + 4 * i);
+    Anchors<1> an;
+    uint32_t gq, sel;
+    {
+        const int y = SH::idle() ? 0 : tid % SH::ROWS, z = zl + SH::ZS * (int)rank;
+        const int n = y + TX * z + SH::R * j, m = (2 * y + 3 * z) % NC;
+        an.an[0] = n;
+        an.rot[0] = 4 * (m ? NC - m : 0);
+        an.base[0] = 4 * (SX * y + SXY * (zl + SH::HALO) + NC * j);
+        // boundary classes; z wraps only where there is one slab
+        const int cy = y == 0 ? 0 : (y == TX - 1 ? 2 : 1), cz = C > 1 ? 1 : zl == 0 ? 0 : (zl == TX - 1 ? 2 : 1);
+        an.cls[0] = 4 * SH::OFFW + 64 * (1 + 3 * cy + 9 * cz);
+        an.xlo[0] = j == 0 ? 0 : -1;
+        an.xhi[0] = j == TX / NC - 1 ? 4 * (NC - 1) : -1;
+        gq = (uint32_t)(n % SH::G);
+        sel = (uint32_t)(n / SH::G) * 0x11u + 0x40u;
+    }
+    auto draw_colours = [&](uint32_t t, uint2 key) {   // of step t, by one warp
+        const uint4 w = philox(make_uint4(t, 0u, (uint32_t)tid | ELP_STREAM_COLOUR, 0u), key);
+        if (tid < SH::NG)
+            reinterpret_cast<uint4*>(S + SH::COLW + 4 * SH::NG * (t & 1))[tid] =
+                make_uint4(4 * bounded(w.x, NC), 4 * bounded(w.y, NC), 4 * bounded(w.z, NC), 4 * bounded(w.w, NC));
+    };
+    const BatchJob& J = a.jobs[a.items[blockIdx.x / C].x];
+    uint32_t* lat = J.lat;
+    uint32_t* rec = J.rec;
+    const uint2 key = make_uint2(J.seed, J.salt);
+    const uint32_t t0 = J.step0 + a.step_base + (a.step_dev ? *a.step_dev : 0u);
+    for (int i = tid; i < SH::R * SH::PLANES; i += SH::THREADS) {
+        const int zp = i / SH::R, xy = i % SH::R;
+        int z = SH::ZS * (int)rank + zp - SH::HALO;
+        z += z < 0 ? TX : 0; z -= z >= TX ? TX : 0;
+        const int idx = xy % TX + SX * (xy / TX) + SXY * zp;
+        uint32_t wv = __ldcg(lat + xy + SH::R * z);
+        if (wv & ELP_LBIT) {
+            const uint32_t chain = wv >> 5;
+            const uint4 rr = __ldcg(reinterpret_cast<const uint4*>(rec + ELP_REC_WORDS * (size_t)chain));
+            wv = (wv & 15) | ((chain + 1) << SH::LSH) | (rr.y << ELP_CSHIFT);
+            S[SH::OFSW + idx] = rr.z;
+        }
+        S[idx] = wv;
+    }
+    if (tid < 32) draw_colours(t0, key);
+    uint32_t rw = own_bytes(t0, 0, gq, sel, key);
+    cp_async_wait_all();
+    if (C > 1) {
+        cluster_arrive();   // every slab is loaded, its mbarriers are set up: words may come
+        cluster_wait();
+    } else {
+        __syncthreads();
+    }
+
+    const uint32_t polls = a.wait_polls ? a.wait_polls : SLAB_POLLS;
+    uint32_t phase = 0;
+    bool alive = true;
+    // End of a substep, in two halves: a warp that sends tells the receiver
+    // how many bytes (having read what it needed of the words that the
+    // receiver may now change), then every thread waits for what this slab
+    // receives and for the CTA.  A thread whose wait gave up sends nothing and
+    // announces nothing any more: unpaced by its neighbours it would arrive at
+    // their mbarriers more often than a phase has room for.
+    auto announce = [&]() {
+        if (sends) {
+            const uint32_t bytes = __reduce_add_sync(0xffffffffu, push.sent);
+            if ((tid & 31) == 0 && alive)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], %1;" ::"r"(push.bar), "r"(bytes) : "memory");
+            push.sent = 0;
+            push.bar ^= 8;
+        }
+    };
+    auto settle = [&](int odd) {
+        if (C > 1 && alive && !wait_parity(bar + 8 * odd, phase, polls)) {
+            alive = false;
+            push.len = 0;
+        }
+        phase ^= odd;
+        __syncthreads();
+    };
+    unsigned long long accepted = 0;
+    for (int st = 0; st < a.nsteps; st++) {
+        const uint32_t t = t0 + (uint32_t)st;
+        uint32_t acc = 0, next = 0;
+        // a test may make one CTA leave after the first step
+        if (C > 1 && st == 1 && (int)blockIdx.x + 1 == a.hold_cta1) {
+            alive = false;
+            break;
+        }
+#pragma unroll 1
+        for (int g = 0; g < SH::NG; g++) {
+            const uint4 c4 = reinterpret_cast<const uint4*>(S + SH::COLW + 4 * SH::NG * (t & 1))[g];
+            acc += slab_substep<SH, NC, 0>(an, rw, (int)c4.x, push);
+            announce();
+            if (g == 0 && tid < 32) draw_colours(t + 1, key);
+            settle(0);
+            acc += slab_substep<SH, NC, 1>(an, rw, (int)c4.y, push);
+            announce();
+            // the next group's bytes while the words are on their way
+            next = own_bytes(g + 1 < SH::NG ? t : t + 1, g + 1 < SH::NG ? g + 1 : 0, gq, sel, key);
+            settle(1);
+            if (!(SH::NSUB % 4 && 4 * g + 2 >= SH::NSUB)) {
+                acc += slab_substep<SH, NC, 2>(an, rw, (int)c4.z, push);
+                announce();
+                settle(0);
+                acc += slab_substep<SH, NC, 3>(an, rw, (int)c4.w, push);
+                announce();
+                settle(1);
+            }
+            rw = next;
+        }
+        accepted += acc;
+        if (C > 1 && !(alive = __syncthreads_and(alive))) break;
+    }
+    if (alive) {
+        for (int i = tid; i < SH::R * SH::ZS; i += SH::THREADS) {
+            const int xy = i % SH::R, idx = xy % TX + SX * (xy / TX) + SXY * (i / SH::R + SH::HALO);
+            const uint32_t site = (uint32_t)(i + SH::R * SH::ZS * (int)rank);
+            uint32_t wv = S[idx];
+            if (wv & SH::LMASK) {
+                const uint32_t chain = ((wv & SH::LMASK) >> SH::LSH) - 1u;
+                *reinterpret_cast<uint4*>(rec + ELP_REC_WORDS * (size_t)chain) =
+                    make_uint4(site, wv >> ELP_CSHIFT, S[SH::OFSW + idx], 0u);
+                wv = (wv & 15) | ELP_LBIT | (chain << 5);
+            }
+            lat[site] = wv;
+        }
+    } else if (tid == 0) {
+        atomicOr(a.error, 4u);
+    }
+    count_accepted(J.acc, accepted);
+    if (C > 1) {
+        cluster_arrive();   // a slab that gave up may still be sent words
+        cluster_wait();
     }
 }
 
@@ -990,6 +1331,56 @@ cudaError_t launch2(const Sweep2Launch* l, Kernel k, std::atomic<int>* per_sm, c
     return cudaLaunchKernelEx(&cfg, k, l->args);
 }
 
+// Whole boxes of rings in C slabs.  Clusters only for melts that have the
+// device to themselves, and as many as are resident at once: a box on 8 SMs
+// takes half the time of one on a single SM, so beside other work it would
+// cost throughput.  cudaErrorNotSupported sends the caller to sweep_box.
+template <int TX, int NC, int SX, int SXY, int C>
+cudaError_t launch_slabs(const Sweep2Launch* l, cudaStream_t s)
+{
+    using SH = elp::Slab<TX, NC, SX, SXY, C>;
+    static std::atomic<int> resident[MAX_DEVICES];   // clusters; 0: not asked yet
+    const auto k = elp::sweep_slabs<TX, NC, SX, SXY, C>;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= MAX_DEVICES) return cudaErrorInvalidDevice;
+    if (C > 1 && !l->alone) return cudaErrorNotSupported;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(l->args.nitems * C));
+    cfg.blockDim = dim3(SH::THREADS);
+    cfg.dynamicSmemBytes = SH::BYTES;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    if (l->check_only) {
+        // chains are numbered in 12 bits; the bound is sweep_box's
+        if (l->max_runs_per_domain > 2048) return cudaErrorNotSupported;
+        static_assert(SH::MAXCHAINS > 2048, "chain numbers");
+        // as in launch2: outside any capture, once per device
+        if (resident[dev].load() < 1) {
+            int n = 1;
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::BYTES);
+            if (e == cudaSuccess && C > 1) e = cudaOccupancyMaxActiveClusters(&n, k, &cfg);
+            if (e != cudaSuccess) return e;
+            if (n < 1) return cudaErrorNotSupported;
+            resident[dev].store(n);
+        }
+    }
+    if (C > 1 && l->args.nitems > resident[dev].load()) return cudaErrorNotSupported;
+    if (l->check_only) {
+        const_cast<Sweep2Launch*>(l)->threads_out = SH::THREADS;
+        const_cast<Sweep2Launch*>(l)->smem_out = SH::BYTES;
+        return cudaSuccess;
+    }
+    if (l->args.nitems < 1) return cudaSuccess;
+    return cudaLaunchKernelEx(&cfg, k, l->args);
+}
+
 template <int TX, int NC, int SX, int SXY, int CAP, int K, bool LIN>
 cudaError_t launch_box(const Sweep2Launch* l, cudaStream_t s)
 {
@@ -1013,6 +1404,21 @@ cudaError_t launch_tiles(const Sweep2Launch* l, cudaStream_t s)
 extern "C" cudaError_t elp_launch_sweep2(const Sweep2Launch* l, cudaStream_t s)
 {
     const elp_geometry& g = l->geom;
+// whole boxes of rings in slabs: edge, colour modulus, strides, slabs
+#define SLABS(X_, NC_, SX_, SXY_, C_)                                                                              \
+    if (g.L == X_ && g.periodic && g.ncol == NC_ && l->sx == SX_ && l->sxy == SXY_ && !l->linear) {                 \
+        const cudaError_t e = launch_slabs<X_, NC_, SX_, SXY_, C_>(l, s);                                           \
+        if (C_ == 1 || e != cudaErrorNotSupported) return e;                                                        \
+    }
+    SLABS(32, 16, 33, 1056, 8)
+    SLABS(30, 15, 30, 900, 6)
+    SLABS(28, 14, 30, 840, 7)
+    SLABS(24, 24, 24, 576, 1)
+    SLABS(22, 22, 22, 484, 1)
+    SLABS(20, 20, 21, 422, 1)
+    SLABS(18, 18, 20, 360, 1)
+    SLABS(16, 16, 16, 256, 1)
+#undef SLABS
     if (l->args.nsteps > 1 && !g.periodic && !l->args.grid_bar) return cudaErrorNotSupported;
 // tiles: edges, colour modulus, shared-memory strides, slot capacity, anchors
 // per thread, min blocks per SM
@@ -1020,41 +1426,36 @@ extern "C" cudaError_t elp_launch_sweep2(const Sweep2Launch* l, cudaStream_t s)
     if (g.tx == X_ && g.ty == Y_ && g.tz == Z_ && !g.periodic && g.ncol == NC_ && l->sx == SX_ && l->sxy == SXY_) \
         return l->linear ? launch_tiles<X_, Y_, Z_, NC_, SX_, SXY_, CAP_, K_, MINB_, true>(l, s)                \
                          : launch_tiles<X_, Y_, Z_, NC_, SX_, SXY_, CAP_, K_, MINB_, false>(l, s);
-// whole boxes: edge, colour modulus, strides, slot capacity, anchors per thread
-#define BOX(X_, NC_, SX_, SXY_, CAP_, K_)                                                                       \
-    if (g.L == X_ && g.periodic && g.ncol == NC_ && l->sx == SX_ && l->sxy == SXY_)                             \
-        return l->linear ? launch_box<X_, NC_, SX_, SXY_, CAP_, K_, true>(l, s)                                 \
-                         : launch_box<X_, NC_, SX_, SXY_, CAP_, K_, false>(l, s);
+// whole boxes: edge, colour modulus, strides, slot capacity, anchors per
+// thread, linear chains
+#define BOX(X_, NC_, SX_, SXY_, CAP_, K_, LIN_)                                                                 \
+    if (g.L == X_ && g.periodic && g.ncol == NC_ && l->sx == SX_ && l->sxy == SXY_ && (l->linear != 0) == LIN_) \
+        return launch_box<X_, NC_, SX_, SXY_, CAP_, K_, LIN_>(l, s);
     TILES(32, 32, 32, 16, 40, 1364, 1792, 2, 1)
     TILES(32, 32, 16, 16, 40, 1364, 1024, 1, 1)
     TILES(32, 16, 16, 16, 40, 724, 1024, 1, 2)
     TILES(16, 16, 16, 16, 24, 444, 512, 1, 3)
     TILES(48, 24, 24, 16, 56, 1456, 2048, 2, 1)
-    BOX(16, 16, 16, 256, 2048, 1)
-    BOX(32, 16, 33, 1056, 2048, 2)
-    BOX(24, 24, 24, 576, 2048, 1)
-#undef BOX
+    BOX(16, 16, 16, 256, 2048, 1, true)
+    BOX(32, 16, 33, 1056, 2048, 2, true)
+    BOX(32, 16, 33, 1056, 2048, 2, false)
+    BOX(24, 24, 24, 576, 2048, 1, true)
 #undef TILES
 // Shapes of rings only (linear chains of these boxes are refused): the even
-// boxes between, and the tiles that boxes of 40, 60, 72, 100, 120 ... take.
-// On the generic kernel a step took 171 us (L = 20), 175 (28), 238 (40) and
-// 251 (72); here 14.9, 24.4, 23.5 and 21.7.
+// boxes between (18 to 22 as one slab, above), and the tiles that boxes of 40,
+// 60, 72, 100, 120 ... take.  On the generic kernel a step took 171 us
+// (L = 20), 175 (28), 238 (40) and 251 (72); here 13.8, 24.0 (14.2 in slabs),
+// 23.5 and 21.7.
 #define TILES(X_, Y_, Z_, NC_, SX_, SXY_, CAP_, K_, MINB_)                                                       \
     if (g.tx == X_ && g.ty == Y_ && g.tz == Z_ && !g.periodic && g.ncol == NC_ && l->sx == SX_ &&                \
         l->sxy == SXY_ && !l->linear)                                                                            \
         return launch_tiles<X_, Y_, Z_, NC_, SX_, SXY_, CAP_, K_, MINB_, false>(l, s);
-#define BOX(X_, NC_, SX_, SXY_, CAP_, K_)                                                                       \
-    if (g.L == X_ && g.periodic && g.ncol == NC_ && l->sx == SX_ && l->sxy == SXY_ && !l->linear)               \
-        return launch_box<X_, NC_, SX_, SXY_, CAP_, K_, false>(l, s);
     TILES(24, 24, 24, 24, 32, 832, 2048, 1, 1)
     TILES(40, 20, 20, 20, 48, 1056, 2048, 1, 1)
     TILES(20, 20, 20, 20, 28, 616, 1024, 1, 2)
-    BOX(18, 18, 20, 360, 2048, 1)
-    BOX(20, 20, 21, 422, 2048, 1)
-    BOX(22, 22, 22, 484, 2048, 1)
-    BOX(26, 13, 26, 676, 2048, 2)
-    BOX(28, 14, 30, 840, 2048, 2)
-    BOX(30, 15, 30, 900, 2048, 2)
+    BOX(26, 13, 26, 676, 2048, 2, false)
+    BOX(28, 14, 30, 840, 2048, 2, false)
+    BOX(30, 15, 30, 900, 2048, 2, false)
 #undef BOX
 #undef TILES
     return cudaErrorNotSupported;

@@ -318,7 +318,7 @@ class Melt:
         return v.value
 
     def debug_waits(self, polls=0, hold_block=-1):
-        """Bound of the grid-barrier waits in tiled multi-step launches (elp_debug_waits)."""
+        """Bound of the waits in multi-step launches (elp_debug_waits)."""
         check(lib().elp_debug_waits(self.h, polls, hold_block))
 
     def close(self):
