@@ -540,7 +540,8 @@ __device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, cons
         if (ok) SW(pY[q]) = nY;
         if (ok && s) SW(pB[q]) = nB;
         if (ok) SW(p[q]) = nP;
-        if (!LIN && ok && ((wP[q] | wB[q] | wY[q]) & SH::LMASK))
+        // (a labelled anchor matters to slot 0 only, where wB is its word)
+        if (!LIN && ok && ((wB[q] | wY[q]) & SH::LMASK))
             follow_label<SH, PER>(p[q], pB[q], pY[q], wP[q], wB[q], wY[q], R[q], E[q]);
         // monomer 0 of a linear chain has no predecessor: no move but its own,
         // below, moves it or joins the front of its run (the branch cost
