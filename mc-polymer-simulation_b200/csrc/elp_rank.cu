@@ -10,18 +10,21 @@
 // quarter or an eighth of them (nodes):
 //   segments  every node walks to the next node of its chain, or to the
 //             chain's last run, and adds up the monomers on the way;
-//   rounds    the nodes jump along their chains by doubling strides (Wyllie's
-//             list ranking), ceil(log2 N) rounds over the nodes alone: each
-//             learns the monomers from its run to the chain's last one and
-//             which run that is;
+//   rounds    the nodes jump along their chains by strides that grow eightfold
+//             (Wyllie's list ranking, there by doubling), ceil(log8 N) rounds
+//             over the nodes alone: each learns the monomers from its run to
+//             the chain's last one and which run that is;
 //   chains    each labelled run checks its chain's length and its last run;
 //   bonds     every node walks its segment again and writes the bonds.
 // A few hops of every chain at once instead of a pass over all sites per
 // round (ranking every site took 10 rounds of 10.5 us at L = 128 and 13 of
-// 110 at L = 256, where its 16 bytes a site leave L2): at L = 128 32 us for
-// the segments, 10 rounds of 5 and 32 for the bonds, and a fetch at L = 256
-// takes 0.82 ms, 1.69 before.  Boxes up to 40^3 do all of it in one kernel on
-// a cluster of CTAs, whose barriers cost less than launches.
+// 110 at L = 256, where its 16 bytes a site leave L2).  The walks and rounds
+// are chains of L2 latencies, and what a launch waits for the one before it
+// costs as much as a small box's round: hence few rounds (by doubling, a
+// checked fetch at L = 64 took 111 us, by eights 91) and launches that are
+// set up while the kernel before them runs (83).  L = 128: 127 us a check by
+// doubling in plain launches, now 88; L = 256: 303, now 247.  Boxes up to 20^3
+// do all of it in one kernel on a cluster of CTAs.
 //
 // The output is the TUV content of cpupol/efpol_io.c:70-77 (start site of
 // monomer 0, N bond codes), the same bytes as walk_kernel writes, and a chain
@@ -102,15 +105,15 @@ __device__ __forceinline__ bool node_run(const RankArgs& a, uint32_t i, Site& s,
         s.v = (int)(uv / (uint32_t)a.L);
         s.t = (int)k * a.q + ((-(2 * s.u + 3 * s.v)) & (a.q - 1));
         if (s.t >= a.L) return false;
-        w = __ldg(a.lat + s.index(a.L));
+        w = a.lat[s.index(a.L)];
         mono = w >> ELP_CSHIFT;
         return w != 0 && !(w & ELP_LBIT);
     }
     const uint32_t p = i - a.heads;
-    const uint4 r = __ldg(reinterpret_cast<const uint4*>(a.rec + ELP_REC_WORDS * (size_t)p));
+    const uint4 r = *reinterpret_cast<const uint4*>(a.rec + ELP_REC_WORDS * (size_t)p);
     if (r.x >= (uint32_t)a.L * a.L * a.L || r.z >= r.y || (a.linear && r.z != 0)) return false;
     s = site_of(r.x, a.L);
-    w = __ldg(a.lat + r.x);
+    w = a.lat[r.x];
     mono = r.y - r.z;
     return (w & ELP_LBIT) && (w >> 5) == p;
 }
@@ -136,7 +139,7 @@ __device__ __forceinline__ void segments(const RankArgs& a, Span sp)
                 if (!elp_valid_bond(b) || hop > a.N) break;
                 Site n = s;
                 n.step(b, a.L);
-                const uint32_t wn = __ldg(a.lat + n.index(a.L));
+                const uint32_t wn = a.lat[n.index(a.L)];
                 if (!wn || (wn & ELP_LBIT)) break;
                 s = n;
                 w = wn;
@@ -151,15 +154,18 @@ __device__ __forceinline__ void segments(const RankArgs& a, Span sp)
     }
 }
 
-// One doubling round: every unfinished node adds its successor's sum and
-// takes its successor's link.
+// One round: every unfinished node takes up to STRIDE - 1 jumps along the links
+// of the round before, each adding that node's sum and taking its link.  (Four
+// at L = 64: 95 us a checked fetch, eight 91, sixteen 91; at L = 256 302, 257
+// and 259 us a check.)
+constexpr int STRIDE = 8;
 __device__ __forceinline__ void round_of(const RankArgs& a, Span sp, int r)
 {
     const uint2* in = a.x[r & 1];
     uint2* out = a.x[(r & 1) ^ 1];
     for (uint32_t i = sp.first; i < a.heads + (uint32_t)a.P; i += sp.count) {
         uint2 e = __ldcg(in + i);
-        if (!(e.x & FIN)) {
+        for (int hop = 1; hop < STRIDE && !(e.x & FIN); hop++) {
             const uint2 f = __ldcg(in + e.x);
             e = make_uint2(f.x, e.y + f.y);
         }
@@ -174,11 +180,11 @@ __device__ __forceinline__ void chain_checks(const RankArgs& a, Span sp, int fin
 {
     for (uint32_t p = sp.first; p < (uint32_t)a.P; p += sp.count) {
         const uint2 e = __ldcg(a.x[fin] + a.heads + p);
-        const uint4 r = __ldg(reinterpret_cast<const uint4*>(a.rec + ELP_REC_WORDS * (size_t)p));
+        const uint4 r = *reinterpret_cast<const uint4*>(a.rec + ELP_REC_WORDS * (size_t)p);
         bool bad = e.x == EMPTY || !(e.x & FIN) || e.y != (a.linear ? (uint32_t)a.N : (uint32_t)a.N - r.z);
         const uint32_t tail = e.x & ~FIN;
         if (!bad) {
-            const uint32_t b = __ldg(a.lat + tail) & 15;
+            const uint32_t b = a.lat[tail] & 15;
             Site s = site_of(tail, a.L);
             s.step(b, a.L);
             bad = a.linear ? b != 15 : (!elp_valid_bond(b) || s.index(a.L) != r.x);
@@ -229,7 +235,7 @@ __device__ __forceinline__ void write_bonds(const RankArgs& a, Span sp, int fin)
         Site s;
         uint32_t w, mono;
         if (!node_run(a, i, s, w, mono)) continue;
-        const uint32_t off = a.linear ? 0u : __ldg(a.rec + ELP_REC_WORDS * (size_t)p + 2);
+        const uint32_t off = a.linear ? 0u : a.rec[ELP_REC_WORDS * (size_t)p + 2];
         long at = (long)a.N - (long)off - (long)e.y;   // place of the run's first monomer
         uint8_t* out = a.bonds ? a.bonds + (size_t)p * a.N : nullptr;
         for (int hop = 0;; hop++) {
@@ -242,7 +248,7 @@ __device__ __forceinline__ void write_bonds(const RankArgs& a, Span sp, int fin)
             if (out) out[at - 1] = (uint8_t)b;
             if (!elp_valid_bond(b) || hop > a.N) break;
             s.step(b, a.L);
-            w = __ldg(a.lat + s.index(a.L));
+            w = a.lat[s.index(a.L)];
             if (!w || (w & ELP_LBIT) || s.is_node(a.q)) break;
             mono = w >> ELP_CSHIFT;
         }
@@ -257,13 +263,13 @@ __device__ __forceinline__ void scan_words(const RankArgs& a, Span sp)
     unsigned long long after = 0, mono = 0;
     uint32_t bad = 0;
     for (uint32_t i = sp.first; i < S; i += sp.count) {
-        const uint32_t w = __ldg(a.lat + i);
+        const uint32_t w = a.lat[i];
         if (!w) continue;
         uint32_t c = w >> ELP_CSHIFT, off = 0;
         if (w & ELP_LBIT) {
             const uint32_t ch = w >> 5;
             uint4 r = make_uint4(EMPTY, 0, 0, 0);
-            if (ch < (uint32_t)a.P) r = __ldg(reinterpret_cast<const uint4*>(a.rec + ELP_REC_WORDS * (size_t)ch));
+            if (ch < (uint32_t)a.P) r = *reinterpret_cast<const uint4*>(a.rec + ELP_REC_WORDS * (size_t)ch);
             if (r.x != i) {
                 bad++;
                 continue;
@@ -304,46 +310,52 @@ __device__ __forceinline__ void all_chain_checks(const RankArgs& a, Span sp, int
     chain_checks(a, sp, fin);
     if (sp.first == 0 && a.flags) a.head->flags = *a.flags;
 }
+// First statement of every kernel here: let the next launch be set up, then
+// wait until the one before has ended and its results are there.  The
+// pointers go through the wait, so that no load moves ahead of it; loads that
+// assume read-only memory (ld.global.nc) have no place in kernels that start
+// before their inputs are written.
+__device__ __forceinline__ void in_turn(RankArgs& a)
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;"
+                 : "+l"(a.lat), "+l"(a.rec), "+l"(a.x[0]), "+l"(a.x[1]), "+l"(a.chain_of), "+l"(a.tail), "+l"(a.head),
+                   "+l"(a.start), "+l"(a.bonds), "+l"(a.status), "+l"(a.flags) :: "memory");
+}
 __global__ void __launch_bounds__(256) rank_segments(RankArgs a, size_t clear)
 {
+    in_turn(a);
     clear_out(a, grid_span(), clear);
     segments(a, grid_span());
 }
-__global__ void __launch_bounds__(256) rank_round(RankArgs a, int r) { round_of(a, grid_span(), r); }
-__global__ void __launch_bounds__(256) rank_chains(RankArgs a, int fin) { all_chain_checks(a, grid_span(), fin); }
+__global__ void __launch_bounds__(256) rank_round(RankArgs a, int r) { in_turn(a); round_of(a, grid_span(), r); }
+__global__ void __launch_bounds__(256) rank_chains(RankArgs a, int fin) { in_turn(a); all_chain_checks(a, grid_span(), fin); }
 __global__ void __launch_bounds__(256) rank_bonds(RankArgs a, int fin)
 {
+    in_turn(a);
     write_bonds(a, grid_span(), fin);
     scan_words(a, grid_span());
 }
 
-// Phases in one launch of one cluster: they hand their results over through
+// All phases in one launch of one cluster: they hand their results over through
 // global memory, and each ends in a cluster barrier, which releases and
 // acquires them; loads that cross it bypass L1.
-__device__ __forceinline__ void cluster_rounds(const RankArgs& a, Span sp, cg::cluster_group& cl, int rounds)
-{
-    for (int r = 0; r < rounds; r++) {
-        round_of(a, sp, r);
-        cl.sync();
-    }
-    all_chain_checks(a, sp, rounds & 1);
-}
 __global__ void __launch_bounds__(1024) rank_cluster(RankArgs a, int rounds, size_t clear)
 {
+    in_turn(a);
     cg::cluster_group cl = cg::this_cluster();
     const Span sp = grid_span();
     clear_out(a, sp, clear);
     segments(a, sp);
+    for (int r = 0; r < rounds; r++) {
+        cl.sync();
+        round_of(a, sp, r);
+    }
     cl.sync();
-    cluster_rounds(a, sp, cl, rounds);
+    all_chain_checks(a, sp, rounds & 1);
     cl.sync();
     write_bonds(a, sp, rounds & 1);
     scan_words(a, sp);
-}
-__global__ void __launch_bounds__(1024) rank_cluster_rounds(RankArgs a, int rounds)
-{
-    cg::cluster_group cl = cg::this_cluster();
-    cluster_rounds(a, grid_span(), cl, rounds);
 }
 
 // Only when the sums disagree: monomers of all runs that reach each chain's
@@ -397,12 +409,11 @@ cudaError_t grow(void** p, size_t* cap, size_t need, size_t* bytes)
     return cudaSuccess;
 }
 
-// Boxes up to this many sites (40^3) are ranked by one cluster, whose barriers
-// replace a dozen launches: a fetch at L = 32 takes 68 us, 95 by launches.
-// At L = 64 eight SMs are too few: 194 us by the cluster, 105 by launches.
-// Up to CLUSTER_NODES nodes (some 56^3 sites) they still do the rounds: L = 48
-// 78 us, 88 by launches (L = 64: 113 and 105).
-constexpr size_t CLUSTER_SITES = (size_t)1 << 16, CLUSTER_NODES = 3 << 14;
+// Boxes up to this many sites (20^3) are ranked by one cluster, whose barriers
+// cost less than launches while its eight SMs are enough: a checked fetch at
+// L = 16 takes 45.7 us (N = 50) and 47 (N = 800), 46.3 and 54 by launches; at
+// L = 32 62 us, 55 by launches.
+constexpr size_t CLUSTER_SITES = (size_t)1 << 13;
 constexpr int CLUSTER = 8;   // CTAs (portable cluster size)
 
 RankArgs rank_args(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear, elp_walk_bufs* b)
@@ -445,31 +456,37 @@ cudaError_t elp_rank_chains(const uint32_t* lat, const uint32_t* rec, int L, int
         a.bonds = nullptr;
         a.start = nullptr;
     }
-    // a chain has at most N runs, so at most N nodes: 2^R >= N strides reach its tail from any of them
+    // a chain has at most N runs, so at most N nodes: STRIDE^R >= N jumps reach its tail from any of them
     int R = 0;
-    while ((1L << R) < (long)N) R++;
+    for (long reach = 1; reach < (long)N; reach *= STRIDE) R++;
     const size_t clear = want_bonds ? b->clear_bytes() : sizeof(elp_chain_head);
-    const int blocks = (int)((nodes + 255) / 256 < 148 * 8 ? (nodes + 255) / 256 : 148 * 8), fin = R & 1;
-    if (S > CLUSTER_SITES) rank_segments<<<blocks, 256, 0, s>>>(a, clear);
-    if (nodes <= CLUSTER_NODES) {
-        cudaLaunchConfig_t cfg = {};
+    const unsigned blocks = (unsigned)((nodes + 255) / 256 < 148 * 8 ? (nodes + 255) / 256 : 148 * 8);
+    const int fin = R & 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (S <= CLUSTER_SITES) {
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = CLUSTER;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
         cfg.gridDim = dim3(CLUSTER);
         cfg.blockDim = dim3(1024);
-        cfg.stream = s;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = CLUSTER;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        if (S <= CLUSTER_SITES) return cudaLaunchKernelEx(&cfg, rank_cluster, a, R, clear);
-        if ((e = cudaLaunchKernelEx(&cfg, rank_cluster_rounds, a, R)) != cudaSuccess) return e;
-    } else {
-        for (int r = 0; r < R; r++) rank_round<<<blocks, 256, 0, s>>>(a, r);
-        rank_chains<<<(P + 255) / 256, 256, 0, s>>>(a, fin);
+        return cudaLaunchKernelEx(&cfg, rank_cluster, a, R, clear);
     }
-    rank_bonds<<<blocks, 256, 0, s>>>(a, fin);
-    return cudaGetLastError();
+    if ((e = cudaLaunchKernelEx(&cfg, rank_segments, a, clear)) != cudaSuccess) return e;
+    for (int r = 0; r < R; r++)
+        if ((e = cudaLaunchKernelEx(&cfg, rank_round, a, r)) != cudaSuccess) return e;
+    cfg.gridDim = dim3((unsigned)((P + 255) / 256));
+    if ((e = cudaLaunchKernelEx(&cfg, rank_chains, a, fin)) != cudaSuccess) return e;
+    cfg.gridDim = dim3(blocks);
+    return cudaLaunchKernelEx(&cfg, rank_bonds, a, fin);
 }
 
 cudaError_t elp_rank_joined(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear, elp_walk_bufs* b,
