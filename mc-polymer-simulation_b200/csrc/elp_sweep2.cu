@@ -1069,6 +1069,9 @@ __global__ void __launch_bounds__(((TY * TZ * (TX / NC) / K) + 31) / 32 * 32, MI
     using SH = Shape<TX, TY, TZ, false, NC, SX, SXY, CAP, K, MINB>;
     uint32_t* S = g_smem;
     const int tid = threadIdx.x;
+    // launches of one step are set up while the one before them runs; what
+    // comes before the wait reads the group's constant tables only
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     load_tables<SH, false>(a);
     for (int i = tid; i < SH::WORDS / 4; i += SH::THREADS)
         reinterpret_cast<uint4*>(S)[i] = make_uint4(HWALL, HWALL, HWALL, HWALL);
@@ -1078,6 +1081,7 @@ __global__ void __launch_bounds__(((TY * TZ * (TX / NC) / K) + 31) / 32 * 32, MI
     Anchors<K> an;
     set_anchors<SH, TX, TY, TZ, false, NC, SX, SXY, K>(an);
     const bool scheduler = tid >= SH::THREADS - 32;   // the warp that sets up the next tile
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t step0 = a.step_base + (a.step_dev ? *a.step_dev : 0u);
 
     unsigned long long accepted = 0;
@@ -1313,14 +1317,17 @@ cudaError_t launch2(const Sweep2Launch* l, Kernel k, std::atomic<int>* per_sm, c
     if (PER || l->args.nsteps <= 1) {
         if (grid > l->nsm * MINB) grid = l->nsm * MINB;
         if (grid < 1) return cudaSuccess;
-        k<<<grid, SH::THREADS, SH::BYTES, s>>>(l->args);
-        return cudaGetLastError();
+        if (PER) {
+            k<<<grid, SH::THREADS, SH::BYTES, s>>>(l->args);
+            return cudaGetLastError();
+        }
     }
     // tiled, several steps: a cooperative launch (every CTA resident, or an
     // error) of at most as many CTAs as fit on the device at once
+    const bool several = l->args.nsteps > 1;
     const int per = per_sm[dev].load();
     if (per < 1) return cudaErrorNotSupported;
-    if (grid > l->nsm * per) grid = l->nsm * per;
+    if (several && grid > l->nsm * per) grid = l->nsm * per;
     if (grid < 1) return cudaSuccess;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
@@ -1328,8 +1335,19 @@ cudaError_t launch2(const Sweep2Launch* l, Kernel k, std::atomic<int>* per_sm, c
     cfg.dynamicSmemBytes = SH::BYTES;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
+    if (several) {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+    } else {
+        // one step: tables and anchors ahead of the previous launch's end (50
+        // steps at L = 128 22.4 -> 19.1 us each, L = 64 15.9 -> 13.5, L = 256
+        // 108.9 -> 106.1), where two launches' CTAs fit side by side or fill
+        // the SMs anyway: in between, the early ones share an SM with their
+        // like later on (125 tiles at L = 80: 16.4 -> 19.0).  Not beside other
+        // groups' work, whose place they would take while they wait.
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = l->alone && (2 * grid <= l->nsm || grid > l->nsm);
+    }
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k, l->args);
