@@ -229,15 +229,18 @@ static bool pageable(const void* p)
 // Chains of up to this many bytes go to pageable host buffers through one
 // copy into pinned memory.  One 315 KB copy and a memcpy take 30 us where
 // three staged copies took 60 (L = 64); above it the memcpy costs more than
-// the driver's own staging.
+// the driver's own staging.  Setting the pinned memory up takes 2 ms and more,
+// so the copies have to have cost that much first.
 constexpr size_t STAGE_BYTES = (size_t)1 << 19;
+constexpr int STAGE_AFTER = 64;
 
 // Wait for the chains queued on the stream and bring them to the host, with
 // the head.
 static elp_status copy_chains(elp_walk_bufs* b, int32_t* start, uint8_t* bonds, elp_chain_head* head, cudaStream_t s)
 {
     const size_t nb = (size_t)b->P * b->N, ns = (size_t)b->P * 12;
-    const bool far = pageable(start) || pageable(bonds), stage = far && b->out_bytes() <= STAGE_BYTES;
+    const bool far = pageable(start) || pageable(bonds);
+    const bool stage = far && b->out_bytes() <= STAGE_BYTES && (b->out_bytes() <= b->cap_h_out || ++b->unstaged > STAGE_AFTER);
     elp_status st = reserve_host_out(b, stage ? b->out_bytes() : sizeof(*head));
     if (st) return st;
     if (stage) {

@@ -52,6 +52,7 @@ struct elp_walk_bufs {
     int32_t* h_status = nullptr;           // pinned host copies of the ring statuses and counters
     unsigned long long* h_cnt = nullptr;
     uint8_t* h_out = nullptr;              // pinned host copy of the head and, of small melts, of all of d_out
+    int unstaged = 0;                      // copies to pageable memory that it would have sped up
     void* d_rank = nullptr;                // list ranking (elp_rank.cu)
     size_t cap_out = 0, cap_rings = 0, cap_sites = 0, cap_obs = 0, cap_h_rings = 0, cap_h_out = 0, cap_rank = 0;
     size_t bytes = 0;
