@@ -117,8 +117,8 @@ elp_status elp_sync(elp_ctx* ctx);
 
 /* Rebuild the rings on the device and copy them to host buffers
  * start[3*P] (int32) and bonds[P*N] (uint8).  Blocking.  The rings are
- * rebuilt by list ranking over all runs at once (boxes up to L = 512; a
- * walk along each ring above).  Returns ELP_ERR_STATE if an earlier launch
+ * rebuilt by list ranking (boxes up to L = 512; a walk along each ring
+ * above).  Returns ELP_ERR_STATE if an earlier launch
  * reported an error (as elp_sync), else ELP_ERR_INTEGRITY if a chain is
  * broken (a bond that is no lattice bond, a run leading to an empty site or
  * into another chain, a wrong monomer count); on either error the buffers'
@@ -128,8 +128,9 @@ elp_status elp_sync(elp_ctx* ctx);
  * (gpupol2/gpupol_cuda.cu:60, gpupol2/oclpol.c:183-376). */
 elp_status elp_fetch_chains(elp_ctx* ctx, int32_t* start, uint8_t* bonds);
 
-/* elp_fetch_chains and elp_check in one pass over the melt (one ring walk,
- * one site scan): the rings go to start[3*P] / bonds[P*N] and the integrity
+/* elp_fetch_chains and elp_check in one pass over the melt (the ranking adds
+ * up all site words beside the chains; a melt it finds amiss is walked and
+ * scanned for the code): the rings go to start[3*P] / bonds[P*N] and the integrity
  * code (0 ok, 3, 4: efpol's codes, cpupol/efpol_io.c:158-211) to *code.
  * With a non-zero code the buffers are unspecified.  The drop-in programs
  * check every dump this way (the reference checks only before and after the

@@ -753,7 +753,7 @@ extern "C" void elp_server_destroy(elp_server* s)
         std::this_thread::sleep_for(std::chrono::milliseconds(5));
     }
     if (s->sched.joinable()) s->sched.join();
-    // the last snapshots: each takes a walk, a check and a file write; give
+    // the last snapshots: each takes a rebuild, a check and a file write; give
     // them a generous bound.  If the I/O threads do not finish in time they
     // are left running with the server's host state (leaked, not freed under
     // them) and only the call returns.

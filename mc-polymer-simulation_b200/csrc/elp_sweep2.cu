@@ -471,7 +471,8 @@ __device__ __noinline__ uint32_t general_substeps(const Anchors<K> an, const uin
 // decide (target, test, the new words' parts), new words come from additions,
 // and the target and next run are stored ahead of the anchor so that a move
 // back into the anchor's run (target = anchor) needs no case of its own.
-// L = 256: 145.8 -> 113.6 us per step together with the tile copy below.
+// L = 256: 145.8 -> 113.6 us per step together with the tile copy below (104.7
+// with the label's branch as it is now).
 // Loads predicated on the lanes that need them cut a tenth of the
 // shared-memory wavefronts but were 3 % slower.
 template <class SH, int K, bool PER, int NC, bool LIN, int KK>
@@ -1062,7 +1063,7 @@ __global__ void __launch_bounds__(Slab<TX, NC, SX, SXY, C>::THREADS, 1) sweep_sl
 // their way, the next tile is set up while this one is stored, and what a
 // tile's load and store need sits in shared memory in between (held in
 // registers it made the substep loop recompute its own).  18.4 us per step
-// now, 23.4 before.
+// then, 23.4 before; 17.5 with the label's branch as it is now.
 template <int TX, int TY, int TZ, int NC, int SX, int SXY, int CAP, int K, int MINB, bool LIN>
 __global__ void __launch_bounds__(((TY * TZ * (TX / NC) / K) + 31) / 32 * 32, MINB) sweep_tiles(BatchLaunch a)
 {
