@@ -302,13 +302,6 @@ elp_status elp_fetch_rings(const uint32_t* lat, const uint32_t* rec, int L, int 
     return ELP_OK;
 }
 
-// The ranked chains hold every monomer of the melt and every site word is in
-// order: integrity code 0.
-static bool all_good(const elp_chain_head& h, int N, int P)
-{
-    return !h.bad && !h.bad_words && h.chain_monomers == h.site_monomers && h.monomers == (unsigned long long)N * P;
-}
-
 elp_status elp_fetch_checked_melt(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear,
                                   const uint32_t* flags, elp_walk_bufs* b, int32_t* start, uint8_t* bonds,
                                   int32_t* code, cudaStream_t s)
@@ -321,7 +314,7 @@ elp_status elp_fetch_checked_melt(const uint32_t* lat, const uint32_t* rec, int 
         elp_chain_head h;
         if ((st = copy_chains(b, start, bonds, &h, s))) return st;
         if ((st = elp_flags_status(h.flags))) return st;
-        if (all_good(h, N, P)) {
+        if (elp_chains_good(h, N, P)) {
             *code = 0;
             return ELP_OK;
         }
@@ -370,7 +363,7 @@ elp_status elp_check_melt(const uint32_t* lat, const uint32_t* rec, int L, int N
         elp_chain_head h;
         memcpy(&h, b->h_out, sizeof(h));
         if ((st = elp_flags_status(h.flags))) return st;
-        if (all_good(h, N, P)) {
+        if (elp_chains_good(h, N, P)) {
             *code = 0;
             return ELP_OK;
         }

@@ -40,6 +40,12 @@ struct elp_chain_head {
     uint32_t pad[6];
 };
 static_assert(sizeof(elp_chain_head) == 64, "the bonds follow 16-byte aligned");
+// The ranked chains hold every monomer of the melt and every site word is in
+// order: integrity code 0.
+inline bool elp_chains_good(const elp_chain_head& h, int N, int P)
+{
+    return !h.bad && !h.bad_words && h.chain_monomers == h.site_monomers && h.monomers == (unsigned long long)N * P;
+}
 
 // Scratch buffers for rebuilding chains on the device.
 struct elp_walk_bufs {

@@ -206,7 +206,8 @@ __global__ void observe_chains(ObsArgs a, const uint8_t* bonds, const int32_t* s
 }  // namespace elp
 
 elp_status elp_observe_melt(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear,
-                            const uint32_t* flags, elp_walk_bufs* b, double* cms_tuv, double* rg2, double* sl, uint64_t* run_hist, int nbins, cudaStream_t s)
+                            const uint32_t* flags, elp_walk_bufs* b, double* cms_tuv, double* rg2, double* sl,
+                            uint64_t* run_hist, int nbins, cudaStream_t s)
 {
     if (nbins < 0 || nbins > ELP_OBS_MAX_BINS)
         return elp_fail(ELP_ERR_ARG, "nbins must be in [0, %d]", ELP_OBS_MAX_BINS);
@@ -227,27 +228,35 @@ elp_status elp_observe_melt(const uint32_t* lat, const uint32_t* rec, int L, int
     ELP_CUDA_TRY(cudaMemsetAsync(a.hist, 0, ELP_OBS_MAX_BINS * sizeof(unsigned long long), s));
     elp_status st = elp_walk_bufs_reserve(b, P, N, 0);
     if (st) return st;
-    // the chains by list ranking, then one pass over their bonds; above the
-    // ranking's box size a walk along each ring
+    const size_t words = (size_t)P * 6 + ELP_OBS_MAX_BINS;
+    std::vector<unsigned long long> o;
+    // the chains by list ranking, then one pass over their bonds
     const cudaError_t re = elp_rank_chains(lat, rec, L, N, P, linear, true, flags, b, s);
-    elp_chain_head h;
-    memset(&h, 0, sizeof(h));
-    if (re != cudaErrorNotSupported) {
+    bool walk = re == cudaErrorNotSupported;
+    if (!walk) {
         ELP_CUDA_TRY(re);
         elp::observe_chains<<<(unsigned)(((size_t)P * 32 + 127) / 128), 128, 0, s>>>(a, b->d_bonds(), b->d_status);
-    } else {
-        elp::observe_kernel<<<(P + 127) / 128, 128, 0, s>>>(a);
-    }
-    ELP_CUDA_TRY(cudaGetLastError());
-    std::vector<unsigned long long> o((size_t)P * 6 + ELP_OBS_MAX_BINS);
-    if (re != cudaErrorNotSupported)
+        ELP_CUDA_TRY(cudaGetLastError());
+        o.resize(words);   // while the device works
+        elp_chain_head h;
         ELP_CUDA_TRY(cudaMemcpyAsync(&h, b->d_out, sizeof(h), cudaMemcpyDeviceToHost, s));
-    ELP_CUDA_TRY(cudaMemcpyAsync(o.data(), a.out, o.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    ELP_CUDA_TRY(cudaStreamSynchronize(s));
-    if (re == cudaErrorNotSupported && flags) {
-        if ((st = elp_device_errors(flags, s))) return st;
-    } else if ((st = elp_flags_status(h.flags))) {
-        return st;
+        ELP_CUDA_TRY(cudaMemcpyAsync(o.data(), a.out, words * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+        ELP_CUDA_TRY(cudaStreamSynchronize(s));
+        if ((st = elp_flags_status(h.flags))) return st;
+        // runs that lead into a chain from outside have written their bonds
+        // into it too: nothing that was summed from them counts
+        walk = !elp_chains_good(h, N, P);
+    }
+    // boxes above the ranking's size, melts it finds amiss: a walk along each
+    // ring from its label, which sees the ring's own runs only
+    if (walk) {
+        o.resize(words);
+        ELP_CUDA_TRY(cudaMemsetAsync(a.hist, 0, ELP_OBS_MAX_BINS * sizeof(unsigned long long), s));
+        elp::observe_kernel<<<(P + 127) / 128, 128, 0, s>>>(a);
+        ELP_CUDA_TRY(cudaGetLastError());
+        ELP_CUDA_TRY(cudaMemcpyAsync(o.data(), a.out, words * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+        ELP_CUDA_TRY(cudaStreamSynchronize(s));
+        if (flags && (st = elp_device_errors(flags, s))) return st;
     }
     for (int p = 0; p < P; p++)
         if (o[6 * (size_t)p + 4] >> 32)
