@@ -226,6 +226,13 @@ elp_status elp_accepted(elp_ctx* ctx, uint64_t* accepted);
  * lets every CTA arrive. */
 elp_status elp_debug_waits(elp_ctx* ctx, uint32_t polls, int32_t hold_block);
 
+/* Test hook: the device scratch of this context's loads, fetches, checks and
+ * observables (given back by this call) may hold no more than `limit` bytes
+ * from now on, as on a device that has no more left (0: no such bound).
+ * Where the rebuild by list ranking finds no room for its 6 to 8 bytes a
+ * site, a walk along each ring gives the same results. */
+elp_status elp_debug_scratch(elp_ctx* ctx, uint64_t limit);
+
 void elp_destroy(elp_ctx* ctx);
 
 /* The 4096-entry transition table (dst1 | dst2<<4 per option), identical to

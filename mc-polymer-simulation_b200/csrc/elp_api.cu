@@ -258,6 +258,16 @@ extern "C" elp_status elp_debug_waits(elp_ctx* c, uint32_t polls, int32_t hold_b
     return ELP_OK;
 }
 
+extern "C" elp_status elp_debug_scratch(elp_ctx* c, uint64_t limit)
+{
+    if (!c) return elp_fail(ELP_ERR_ARG, "null context");
+    ELP_CUDA_TRY(cudaSetDevice(c->device));
+    ELP_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    elp_walk_bufs_free(&c->wb);
+    c->wb.limit = (size_t)limit;
+    return ELP_OK;
+}
+
 extern "C" elp_status elp_fetch_chains(elp_ctx* c, int32_t* start, uint8_t* bonds)
 {
     if (!c || !start || !bonds) return elp_fail(ELP_ERR_ARG, "null argument");

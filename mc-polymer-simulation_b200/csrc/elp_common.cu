@@ -151,40 +151,48 @@ void elp_walk_bufs_free(elp_walk_bufs* b)
     *b = elp_walk_bufs();
 }
 
+static cudaError_t scratch_alloc(elp_walk_bufs* b, void** p, size_t* cap, size_t n)
+{
+    if (b->limit && b->bytes + n > b->limit) return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMalloc(p, n);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return e;
+    }
+    *cap = n;
+    b->bytes += n;
+    return cudaSuccess;
+}
+
+static void scratch_free(elp_walk_bufs* b, void** p, size_t* cap)
+{
+    cudaFree(*p);
+    *p = nullptr;
+    b->bytes -= *cap;
+    *cap = 0;
+}
+
+cudaError_t elp_scratch_grow(elp_walk_bufs* b, void** p, size_t* cap, size_t need)
+{
+    if (need <= *cap) return cudaSuccess;
+    const size_t more = std::max(need, *cap + *cap / 2);
+    scratch_free(b, p, cap);
+    cudaError_t e = scratch_alloc(b, p, cap, more);
+    if (e == cudaErrorMemoryAllocation && more > need) e = scratch_alloc(b, p, cap, need);
+    if (e == cudaErrorMemoryAllocation && b->cap_rank) {
+        scratch_free(b, &b->d_rank, &b->cap_rank);
+        e = scratch_alloc(b, p, cap, need);
+    }
+    return e;
+}
+
 elp_status elp_walk_bufs_reserve(elp_walk_bufs* b, int P, int N, size_t sites)
 {
     b->P = P;
     b->N = N;
-    if (b->out_bytes() > b->cap_out) {
-        // grow by half at least: a batch's members come in any order of size,
-        // and every growth synchronises the device
-        const size_t need = std::max(b->out_bytes(), b->cap_out + b->cap_out / 2);
-        cudaFree(b->d_out);
-        b->d_out = nullptr;
-        b->bytes -= b->cap_out;
-        b->cap_out = 0;
-        ELP_CUDA_TRY(cudaMalloc((void**)&b->d_out, need));
-        b->cap_out = need;
-        b->bytes += need;
-    }
-    if ((size_t)P > b->cap_rings) {
-        cudaFree(b->d_status);
-        b->d_status = nullptr;
-        b->bytes -= b->cap_rings * 4;
-        b->cap_rings = 0;
-        ELP_CUDA_TRY(cudaMalloc((void**)&b->d_status, (size_t)P * sizeof(int32_t)));
-        b->cap_rings = (size_t)P;
-        b->bytes += (size_t)P * 4;
-    }
-    if (sites > b->cap_sites) {
-        cudaFree(b->d_visit);
-        b->d_visit = nullptr;
-        b->bytes -= b->cap_sites * 4;
-        b->cap_sites = 0;
-        ELP_CUDA_TRY(cudaMalloc((void**)&b->d_visit, sites * sizeof(uint32_t)));
-        b->cap_sites = sites;
-        b->bytes += sites * 4;
-    }
+    ELP_CUDA_TRY(elp_scratch_grow(b, (void**)&b->d_out, &b->cap_out, b->out_bytes()));
+    ELP_CUDA_TRY(elp_scratch_grow(b, (void**)&b->d_status, &b->cap_status, (size_t)P * sizeof(int32_t)));
+    ELP_CUDA_TRY(elp_scratch_grow(b, (void**)&b->d_visit, &b->cap_visit, sites * sizeof(uint32_t)));
     if (sites && !b->d_cnt) ELP_CUDA_TRY(cudaMalloc((void**)&b->d_cnt, 8 * sizeof(unsigned long long)));
     return ELP_OK;
 }
@@ -270,9 +278,9 @@ elp_status elp_fetch_rings(const uint32_t* lat, const uint32_t* rec, int L, int 
     elp_status st = elp_walk_bufs_reserve(b, P, N, 0);
     if (st) return st;
     // list ranking: every chain's segments at once; the chain walk (one
-    // ring's latency) for boxes too large for its scratch
+    // ring's latency) for boxes above its size or without room for its scratch
     const cudaError_t re = elp_rank_chains(lat, rec, L, N, P, linear, true, flags, b, s);
-    if (re != cudaErrorNotSupported) {
+    if (!elp_must_walk(re)) {
         ELP_CUDA_TRY(re);
         elp_chain_head h;
         if ((st = copy_chains(b, start, bonds, &h, s))) return st;
@@ -309,7 +317,7 @@ elp_status elp_fetch_checked_melt(const uint32_t* lat, const uint32_t* rec, int 
     elp_status st = elp_walk_bufs_reserve(b, P, N, 0);
     if (st) return st;
     const cudaError_t re = elp_rank_chains(lat, rec, L, N, P, linear, true, flags, b, s);
-    if (re != cudaErrorNotSupported) {
+    if (!elp_must_walk(re)) {
         ELP_CUDA_TRY(re);
         elp_chain_head h;
         if ((st = copy_chains(b, start, bonds, &h, s))) return st;
@@ -319,7 +327,7 @@ elp_status elp_fetch_checked_melt(const uint32_t* lat, const uint32_t* rec, int 
             return ELP_OK;
         }
     }
-    // something is wrong (or the box too large to rank): the walk and the
+    // something is wrong (or the melt could not be ranked): the walk and the
     // site scan with visit counters tell efpol's codes apart
     const size_t S = (size_t)L * L * L;
     if ((st = elp_walk_bufs_reserve(b, P, N, S)) || (st = reserve_host_status(b, P))) return st;
@@ -355,7 +363,7 @@ elp_status elp_check_melt(const uint32_t* lat, const uint32_t* rec, int L, int N
     elp_status st = elp_walk_bufs_reserve(b, P, N, 0);
     if (st) return st;
     const cudaError_t re = elp_rank_chains(lat, rec, L, N, P, linear, false, flags, b, s);
-    if (re != cudaErrorNotSupported) {
+    if (!elp_must_walk(re)) {
         ELP_CUDA_TRY(re);
         if ((st = reserve_host_out(b, sizeof(elp_chain_head)))) return st;
         ELP_CUDA_TRY(cudaMemcpyAsync(b->h_out, b->d_out, sizeof(elp_chain_head), cudaMemcpyDeviceToHost, s));

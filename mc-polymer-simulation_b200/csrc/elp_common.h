@@ -60,8 +60,10 @@ struct elp_walk_bufs {
     uint8_t* h_out = nullptr;              // pinned host copy of the head and, of small melts, of all of d_out
     int unstaged = 0;                      // copies to pageable memory that it would have sped up
     void* d_rank = nullptr;                // list ranking (elp_rank.cu)
-    size_t cap_out = 0, cap_rings = 0, cap_sites = 0, cap_obs = 0, cap_h_rings = 0, cap_h_out = 0, cap_rank = 0;
-    size_t bytes = 0;
+    size_t cap_out = 0, cap_status = 0, cap_visit = 0, cap_obs = 0, cap_rank = 0;   // device bytes
+    size_t cap_h_rings = 0, cap_h_out = 0;
+    size_t bytes = 0;                      // device bytes held
+    size_t limit = 0;                      // test hook: no more than these (0: what the device has)
 
     static size_t bond_bytes(int P, int N) { return ((size_t)P * N + 15) & ~(size_t)15; }
     elp_chain_head* head() const { return reinterpret_cast<elp_chain_head*>(d_out); }
@@ -71,6 +73,12 @@ struct elp_walk_bufs {
     size_t out_bytes() const { return clear_bytes() + (size_t)P * 12; }
 };
 void elp_walk_bufs_free(elp_walk_bufs* b);
+// Grow one of b's device buffers (*p, *cap bytes) to `need` bytes, by half at
+// least where the device has room for that: a batch's members come in any
+// order of size, and every growth synchronises the device.  The old contents
+// are lost.  Where there is no room the ranking's scratch is given up first
+// (its callers can walk); cudaErrorMemoryAllocation leaves the buffer empty.
+cudaError_t elp_scratch_grow(elp_walk_bufs* b, void** p, size_t* cap, size_t need);
 // Lay the scratch out for P chains of N (and grow it), with `sites` visit
 // counters.
 elp_status elp_walk_bufs_reserve(elp_walk_bufs* b, int P, int N, size_t sites);
@@ -89,9 +97,14 @@ constexpr size_t ELP_RANK_MAX_SITES = (size_t)1 << 27;
 // Chains of one melt into b's head, bonds, start and statuses by list ranking
 // (elp_rank.cu), stream-ordered; without bonds the checks alone.  `flags`
 // (or null): device error flags to put into the head.  cudaErrorNotSupported
-// (nothing launched) above ELP_RANK_MAX_SITES sites.
+// (nothing launched) above ELP_RANK_MAX_SITES sites, cudaErrorMemoryAllocation
+// (nothing launched) if its scratch finds no room: the callers then walk.
 cudaError_t elp_rank_chains(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear, bool want_bonds,
                             const uint32_t* flags, elp_walk_bufs* b, cudaStream_t s);
+inline bool elp_must_walk(cudaError_t ranked)
+{
+    return ranked == cudaErrorNotSupported || ranked == cudaErrorMemoryAllocation;
+}
 // After it, where the head's sums disagree or a chain is broken: also find
 // the chains that other runs lead into.
 cudaError_t elp_rank_joined(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear, elp_walk_bufs* b,

@@ -212,27 +212,20 @@ elp_status elp_observe_melt(const uint32_t* lat, const uint32_t* rec, int L, int
     if (nbins < 0 || nbins > ELP_OBS_MAX_BINS)
         return elp_fail(ELP_ERR_ARG, "nbins must be in [0, %d]", ELP_OBS_MAX_BINS);
     if (run_hist && nbins < 1) return elp_fail(ELP_ERR_ARG, "run_hist needs nbins >= 1");
-    const size_t need = (size_t)P * 6 + ELP_OBS_MAX_BINS;
-    if (need > b->cap_obs) {
-        cudaFree(b->d_obs);
-        b->d_obs = nullptr;
-        ELP_CUDA_TRY(cudaMalloc((void**)&b->d_obs, need * sizeof(unsigned long long)));
-        b->bytes += (need - b->cap_obs) * sizeof(unsigned long long);
-        b->cap_obs = need;
-    }
+    const size_t words = (size_t)P * 6 + ELP_OBS_MAX_BINS;
+    ELP_CUDA_TRY(elp_scratch_grow(b, (void**)&b->d_obs, &b->cap_obs, words * sizeof(unsigned long long)));
     elp::ObsArgs a;
     a.lat = lat; a.rec = rec; a.L = L; a.N = N; a.P = P; a.linear = linear;
     a.nbins = nbins > 0 ? nbins : 1;
     a.out = b->d_obs;
     a.hist = b->d_obs + (size_t)P * 6;
     ELP_CUDA_TRY(cudaMemsetAsync(a.hist, 0, ELP_OBS_MAX_BINS * sizeof(unsigned long long), s));
-    elp_status st = elp_walk_bufs_reserve(b, P, N, 0);
-    if (st) return st;
-    const size_t words = (size_t)P * 6 + ELP_OBS_MAX_BINS;
     std::vector<unsigned long long> o;
     // the chains by list ranking, then one pass over their bonds
-    const cudaError_t re = elp_rank_chains(lat, rec, L, N, P, linear, true, flags, b, s);
-    bool walk = re == cudaErrorNotSupported;
+    elp_status st = elp_walk_bufs_reserve(b, P, N, 0);
+    if (st && st != ELP_ERR_NOMEM) return st;
+    const cudaError_t re = st ? cudaErrorMemoryAllocation : elp_rank_chains(lat, rec, L, N, P, linear, true, flags, b, s);
+    bool walk = elp_must_walk(re);
     if (!walk) {
         ELP_CUDA_TRY(re);
         elp::observe_chains<<<(unsigned)(((size_t)P * 32 + 127) / 128), 128, 0, s>>>(a, b->d_bonds(), b->d_status);
@@ -247,8 +240,9 @@ elp_status elp_observe_melt(const uint32_t* lat, const uint32_t* rec, int L, int
         // into it too: nothing that was summed from them counts
         walk = !elp_chains_good(h, N, P);
     }
-    // boxes above the ranking's size, melts it finds amiss: a walk along each
-    // ring from its label, which sees the ring's own runs only
+    // boxes above the ranking's size, no room for its scratch (the walk needs
+    // none), melts it finds amiss: a walk along each ring from its label, which
+    // sees the ring's own runs only
     if (walk) {
         o.resize(words);
         ELP_CUDA_TRY(cudaMemsetAsync(a.hist, 0, ELP_OBS_MAX_BINS * sizeof(unsigned long long), s));

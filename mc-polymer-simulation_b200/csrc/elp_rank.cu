@@ -394,21 +394,6 @@ __global__ void rank_totals(RankArgs a, const uint32_t* total)
     if (total[p] != (uint32_t)a.N - off) chain_bad(a, (uint32_t)p);
 }
 
-cudaError_t grow(void** p, size_t* cap, size_t need, size_t* bytes)
-{
-    if (need <= *cap) return cudaSuccess;
-    if (need < *cap + *cap / 2) need = *cap + *cap / 2;   // as elp_walk_bufs_reserve
-    cudaFree(*p);
-    *p = nullptr;
-    *bytes -= *cap;
-    *cap = 0;
-    const cudaError_t e = cudaMalloc(p, need);
-    if (e != cudaSuccess) return e;
-    *cap = need;
-    *bytes += need;
-    return cudaSuccess;
-}
-
 // Boxes up to this many sites (20^3) are ranked by one cluster, whose barriers
 // cost less than launches while its eight SMs are enough: a checked fetch at
 // L = 16 takes 45.7 us (N = 50) and 47 (N = 800), 46.3 and 54 by launches; at
@@ -448,7 +433,7 @@ cudaError_t elp_rank_chains(const uint32_t* lat, const uint32_t* rec, int L, int
     if (S > ELP_RANK_MAX_SITES || P <= 0) return cudaErrorNotSupported;
     const int q = S <= ((size_t)1 << 22) ? 4 : 8;
     const size_t nodes = (size_t)((L + q - 1) / q) * L * L + P;
-    cudaError_t e = grow(&b->d_rank, &b->cap_rank, nodes * 16 + S * 4 + (size_t)P * 4, &b->bytes);
+    cudaError_t e = elp_scratch_grow(b, &b->d_rank, &b->cap_rank, nodes * 16 + S * 4 + (size_t)P * 4);
     if (e != cudaSuccess) return e;
     RankArgs a = rank_args(lat, rec, L, N, P, linear, b);
     a.flags = flags;

@@ -41,7 +41,7 @@ class Info(C.Structure):
 EXPORTED = [
     "elp_default_spec", "elp_create", "elp_init_melt", "elp_load_chains", "elp_load_tuv", "elp_run",
     "elp_run_timed", "elp_stream", "elp_sync", "elp_fetch_chains", "elp_fetch_checked", "elp_write_tuv", "elp_check", "elp_get_info",
-    "elp_get_state", "elp_set_state", "elp_accepted", "elp_debug_waits", "elp_time_factor", "elp_destroy", "elp_transition_table",
+    "elp_get_state", "elp_set_state", "elp_accepted", "elp_debug_waits", "elp_debug_scratch", "elp_time_factor", "elp_destroy", "elp_transition_table",
     "elp_format_tuv", "elp_status_string", "elp_last_error",
     "elp_batch_create", "elp_batch_size", "elp_batch_init_melts", "elp_batch_load_chains", "elp_batch_run",
     "elp_batch_run_timed", "elp_batch_sync", "elp_batch_fetch_chains", "elp_batch_get_state", "elp_batch_check",
@@ -84,6 +84,7 @@ def lib():
         "elp_set_state": (i32, [vp, vp, vp, u64]),
         "elp_accepted": (i32, [vp, vp]),
         "elp_debug_waits": (i32, [vp, u32, i32]),
+        "elp_debug_scratch": (i32, [vp, u64]),
         "elp_time_factor": (C.c_double, [i32, i32, i32, i32]),
         "elp_destroy": (None, [vp]),
         "elp_transition_table": (i32, [vp]),
@@ -320,6 +321,10 @@ class Melt:
     def debug_waits(self, polls=0, hold_block=-1):
         """Bound of the waits in multi-step launches (elp_debug_waits)."""
         check(lib().elp_debug_waits(self.h, polls, hold_block))
+
+    def debug_scratch(self, limit=0):
+        """Bound of the context's device scratch in bytes (elp_debug_scratch)."""
+        check(lib().elp_debug_scratch(self.h, limit))
 
     def close(self):
         if getattr(self, "h", None) and self.h.value:
