@@ -285,7 +285,7 @@ elp_status elp_fetch_rings(const uint32_t* lat, const uint32_t* rec, int L, int 
         elp_chain_head h;
         if ((st = copy_chains(b, start, bonds, &h, s))) return st;
         if ((st = elp_flags_status(h.flags))) return st;
-        if (h.bad || h.chain_monomers != h.site_monomers) {
+        if (h.bad || h.bad_words || h.chain_monomers != h.site_monomers) {
             ELP_CUDA_TRY(elp_rank_joined(lat, rec, L, N, P, linear, b, s));
             ELP_CUDA_TRY(cudaMemcpyAsync(&h, b->d_out, sizeof(h), cudaMemcpyDeviceToHost, s));
             ELP_CUDA_TRY(cudaStreamSynchronize(s));

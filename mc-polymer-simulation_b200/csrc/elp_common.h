@@ -105,8 +105,8 @@ inline bool elp_must_walk(cudaError_t ranked)
 {
     return ranked == cudaErrorNotSupported || ranked == cudaErrorMemoryAllocation;
 }
-// After it, where the head's sums disagree or a chain is broken: also find
-// the chains that other runs lead into.
+// After it, where the head's sums disagree, a word breaks a rule or a chain is
+// broken: also find the chains that other runs lead into.
 cudaError_t elp_rank_joined(const uint32_t* lat, const uint32_t* rec, int L, int N, int P, int linear, elp_walk_bufs* b,
                             cudaStream_t s);
 // Rebuild rings (start[3P], bonds[P*N]) of one melt into host buffers.  Error

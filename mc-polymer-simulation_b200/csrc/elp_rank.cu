@@ -358,8 +358,10 @@ __global__ void __launch_bounds__(1024) rank_cluster(RankArgs a, int rounds, siz
     scan_words(a, sp);
 }
 
-// Only when the sums disagree: monomers of all runs that reach each chain's
-// tail, one run per thread, and the chains with more than their own.
+// Only when the sums disagree or a word breaks a rule: monomers of all runs that
+// reach each chain's tail, one run per thread, and the chains with more than
+// their own.  A word of no monomers (an empty run, a label of no chain) that
+// reaches a tail makes its chain bad by itself.
 __global__ void __launch_bounds__(256) rank_joined(RankArgs a, uint32_t* total)
 {
     const uint32_t S = (uint32_t)a.L * a.L * a.L;
@@ -369,9 +371,8 @@ __global__ void __launch_bounds__(256) rank_joined(RankArgs a, uint32_t* total)
         uint32_t mono = w >> ELP_CSHIFT;
         if (w & ELP_LBIT) {
             const uint32_t ch = w >> 5;
-            if (ch >= (uint32_t)a.P) continue;
             const uint32_t* r = a.rec + ELP_REC_WORDS * (size_t)ch;
-            mono = r[2] < r[1] ? r[1] - r[2] : 0u;
+            mono = ch < (uint32_t)a.P && r[2] < r[1] ? r[1] - r[2] : 0u;
         }
         Site s = site_of(i, a.L);
         uint32_t tail = i;
@@ -383,7 +384,9 @@ __global__ void __launch_bounds__(256) rank_joined(RankArgs a, uint32_t* total)
             tail = s.index(a.L);
         }
         const uint32_t p = a.chain_of[tail];
-        if (p < (uint32_t)a.P && a.tail[p] == tail) atomicAdd(&total[p], mono);
+        if (p >= (uint32_t)a.P || a.tail[p] != tail) continue;
+        if (mono) atomicAdd(&total[p], mono);
+        else chain_bad(a, p);
     }
 }
 __global__ void rank_totals(RankArgs a, const uint32_t* total)
