@@ -213,7 +213,6 @@ static elp_status reserve_host_status(elp_walk_bufs* b, int P)
 static elp_status reserve_host_out(elp_walk_bufs* b, size_t need)
 {
     if (need > b->cap_h_out) {
-        if (b->cap_h_out) need = std::max(need, 2 * b->cap_h_out);
         cudaFreeHost(b->h_out);
         b->h_out = nullptr;
         b->cap_h_out = 0;
@@ -238,7 +237,8 @@ static bool pageable(const void* p)
 // copy into pinned memory.  One 315 KB copy and a memcpy take 30 us where
 // three staged copies took 60 (L = 64); above it the memcpy costs more than
 // the driver's own staging.  Setting the pinned memory up takes 2 ms and more,
-// so the copies have to have cost that much first.
+// so the copies have to have cost that much first; it is set up once, at this
+// size (a batch's members come in any order of size).
 constexpr size_t STAGE_BYTES = (size_t)1 << 19;
 constexpr int STAGE_AFTER = 64;
 
@@ -248,9 +248,14 @@ static elp_status copy_chains(elp_walk_bufs* b, int32_t* start, uint8_t* bonds, 
 {
     const size_t nb = (size_t)b->P * b->N, ns = (size_t)b->P * 12;
     const bool far = pageable(start) || pageable(bonds);
-    const bool stage = far && b->out_bytes() <= STAGE_BYTES && (b->out_bytes() <= b->cap_h_out || ++b->unstaged > STAGE_AFTER);
-    elp_status st = reserve_host_out(b, stage ? b->out_bytes() : sizeof(*head));
-    if (st) return st;
+    bool stage = far && b->out_bytes() <= STAGE_BYTES && (b->cap_h_out >= STAGE_BYTES || ++b->unstaged > STAGE_AFTER);
+    elp_status st = ELP_OK;
+    if (stage && reserve_host_out(b, STAGE_BYTES)) {
+        cudaGetLastError();   // no room for it: the driver stages
+        stage = false;
+        b->unstaged = 0;
+    }
+    if (!stage && (st = reserve_host_out(b, sizeof(*head)))) return st;
     if (stage) {
         ELP_CUDA_TRY(cudaMemcpyAsync(b->h_out, b->d_out, b->out_bytes(), cudaMemcpyDeviceToHost, s));
         ELP_CUDA_TRY(cudaStreamSynchronize(s));
