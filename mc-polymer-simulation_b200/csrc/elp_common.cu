@@ -143,10 +143,16 @@ elp_status elp_flags_status(uint32_t flags)
     return ELP_OK;
 }
 
+static void device_free(const elp_walk_bufs* b, void* p)
+{
+    if (b->pooled && p) cudaFreeAsync(p, b->pooled);
+    else cudaFree(p);
+}
+
 void elp_walk_bufs_free(elp_walk_bufs* b)
 {
-    cudaFree(b->d_out); cudaFree(b->d_status); cudaFree(b->d_visit); cudaFree(b->d_cnt);
-    cudaFree(b->d_obs); cudaFree(b->d_rank);
+    for (void* p : {(void*)b->d_out, (void*)b->d_status, (void*)b->d_visit, (void*)b->d_obs, b->d_rank}) device_free(b, p);
+    cudaFree(b->d_cnt);
     cudaFreeHost(b->h_status); cudaFreeHost(b->h_cnt); cudaFreeHost(b->h_out);
     *b = elp_walk_bufs();
 }
@@ -154,7 +160,7 @@ void elp_walk_bufs_free(elp_walk_bufs* b)
 static cudaError_t scratch_alloc(elp_walk_bufs* b, void** p, size_t* cap, size_t n)
 {
     if (b->limit && b->bytes + n > b->limit) return cudaErrorMemoryAllocation;
-    const cudaError_t e = cudaMalloc(p, n);
+    const cudaError_t e = b->pooled ? cudaMallocAsync(p, n, b->pooled) : cudaMalloc(p, n);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return e;
@@ -166,7 +172,7 @@ static cudaError_t scratch_alloc(elp_walk_bufs* b, void** p, size_t* cap, size_t
 
 static void scratch_free(elp_walk_bufs* b, void** p, size_t* cap)
 {
-    cudaFree(*p);
+    device_free(b, *p);
     *p = nullptr;
     b->bytes -= *cap;
     *cap = 0;

@@ -64,6 +64,7 @@ struct elp_walk_bufs {
     size_t cap_h_rings = 0, cap_h_out = 0;
     size_t bytes = 0;                      // device bytes held
     size_t limit = 0;                      // test hook: no more than these (0: what the device has)
+    cudaStream_t pooled = nullptr;         // set: device buffers from the device's memory pool, in this stream's order
 
     static size_t bond_bytes(int P, int N) { return ((size_t)P * N + 15) & ~(size_t)15; }
     elp_chain_head* head() const { return reinterpret_cast<elp_chain_head*>(d_out); }
