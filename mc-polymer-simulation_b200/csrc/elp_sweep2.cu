@@ -1466,6 +1466,16 @@ extern "C" cudaError_t elp_launch_sweep2(const Sweep2Launch* l, cudaStream_t s)
     TILES(32, 32, 32, 16, 40, 1364, 1792, 2, 1)
     TILES(32, 32, 16, 16, 40, 1364, 1024, 1, 1)
     TILES(32, 16, 16, 16, 40, 724, 1024, 1, 2)
+    // 16^3: three CTAs an SM leave the compiler registers for a faster kernel
+    // (one box of L = 64: 12.0 us per step, 12.9 with four), but four take 512
+    // tiles in one round (8 boxes of L = 64 22.8 against 31.1, L = 128 21.2
+    // against 29.0).  A round's time is as the CTAs in it (16 and 21.4 us): four
+    // where their rounds hold fewer slots in all (729 tiles, L = 144: 28.8 with
+    // three, 39.5 with four; 2304 tiles: 92.1 and 85.2; 3072: 108 and 124).
+    auto slots = [&](int per_sm) { return (l->args.nitems + l->nsm * per_sm - 1) / (l->nsm * per_sm) * per_sm; };
+    if (slots(4) < slots(3)) {
+        TILES(16, 16, 16, 16, 24, 444, 512, 1, 4)
+    }
     TILES(16, 16, 16, 16, 24, 444, 512, 1, 3)
     TILES(48, 24, 24, 16, 56, 1456, 2048, 2, 1)
     BOX(16, 16, 16, 256, 2048, 1, true)
