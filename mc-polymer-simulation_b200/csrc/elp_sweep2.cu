@@ -645,6 +645,31 @@ __device__ __forceinline__ void load_tables(const BatchLaunch& a)
     for (int i = threadIdx.x; i < 64; i += SH::THREADS) g_smem[SH::HTABW + i] = a.table[960 + i];
 }
 
+// Words i < N of a whole box into shared memory, strided over the CTA: word i
+// comes from src(i) and goes to word at(i); labelled(word, place) is called for
+// the labelled ones, once a thread has copied all of its words.  (With a branch
+// for them between the loads, and a record's latency behind it, a launch of one
+// step took 18.8 us at L = 16 and 22.5 at L = 18, now 15.1 and 20.5.)
+template <int N, int THREADS, class Src, class At, class Labelled>
+__device__ __forceinline__ void load_words(Src src, At at, Labelled labelled)
+{
+    static_assert((N + THREADS - 1) / THREADS <= 32, "a bit for each of a thread's words");
+    const int tid = threadIdx.x;
+    uint32_t mask = 0;
+#pragma unroll 8
+    for (int k = 0; k < (N + THREADS - 1) / THREADS; k++) {
+        const int i = tid + k * THREADS;
+        const bool in = N % THREADS == 0 || i < N;
+        const uint32_t wv = in ? __ldcg(src(i)) : 0u;
+        if (in) g_smem[at(i)] = wv;
+        mask |= wv & ELP_LBIT ? 1u << k : 0u;
+    }
+    for (; mask; mask &= mask - 1) {
+        const int idx = at(tid + (__ffs(mask) - 1) * THREADS);
+        labelled(g_smem[idx], idx);
+    }
+}
+
 // Whole boxes of linear chains, and of rings where sweep_slabs below does not
 // run: each CTA holds one melt for all steps of the launch.
 //
@@ -671,12 +696,9 @@ __global__ void __launch_bounds__(((TX * TX * (TX / NC) / K) + 31) / 32 * 32, 1)
         __syncthreads();   // the previous melt's words and slots have been read
         if (tid == 0) g_smem[SH::NSLW] = 0;
         __syncthreads();
-        for (int i = tid; i < SITES; i += SH::THREADS) {
-            const int idx = i % TX + SX * (i / TX % TX) + SXY * (i / (TX * TX));
-            const uint32_t wv = __ldcg(lat + i);
-            S[idx] = wv;
-            if (wv & ELP_LBIT) claim_slot<SH>(wv, idx);
-        }
+        load_words<SITES, SH::THREADS>([&](int i) { return lat + i; },
+                                       [](int i) { return i % TX + SX * (i / TX % TX) + SXY * (i / (TX * TX)); },
+                                       [](uint32_t wv, int idx) { claim_slot<SH>(wv, idx); });
         cp_async_wait_all();
         __syncthreads();
         const uint32_t ns = g_smem[SH::NSLW];
@@ -918,6 +940,30 @@ __global__ void __launch_bounds__(Slab<TX, NC, SX, SXY, C>::THREADS, 1) sweep_sl
     for (int i = tid; i < SH::TABS / 4; i += SH::THREADS) cp_async16(S + SH::TABW + 4 * i, a.moves + 4 * i);
     for (int i = tid; i < ELP_MOVE_ENTRIES / 4; i += SH::THREADS)
         cp_async16(S + SH::DTABW + 4 * i, a.moves + SH::TABS + 4 * i);
+    auto draw_colours = [&](uint32_t t, uint2 key) {   // of step t, by one warp
+        const uint4 w = philox(make_uint4(t, 0u, (uint32_t)tid | ELP_STREAM_COLOUR, 0u), key);
+        if (tid < SH::NG)
+            reinterpret_cast<uint4*>(S + SH::COLW + 4 * SH::NG * (t & 1))[tid] =
+                make_uint4(4 * bounded(w.x, NC), 4 * bounded(w.y, NC), 4 * bounded(w.z, NC), 4 * bounded(w.w, NC));
+    };
+    const BatchJob& J = a.jobs[a.items[blockIdx.x / C].x];
+    uint32_t* lat = J.lat;
+    uint32_t* rec = J.rec;
+    const uint2 key = make_uint2(J.seed, J.salt);
+    const uint32_t t0 = J.step0 + a.step_base + (a.step_dev ? *a.step_dev : 0u);
+    load_words<SH::R * SH::PLANES, SH::THREADS>(
+        [&](int i) {
+            int z = SH::ZS * (int)rank + i / SH::R - SH::HALO;
+            z += z < 0 ? TX : 0; z -= z >= TX ? TX : 0;
+            return lat + i % SH::R + SH::R * z;
+        },
+        [](int i) { return i % TX + SX * (i / TX % TX) + SXY * (i / SH::R); },
+        [&](uint32_t wv, int idx) {
+            const uint32_t chain = wv >> 5;
+            const uint4 rr = __ldcg(reinterpret_cast<const uint4*>(rec + ELP_REC_WORDS * (size_t)chain));
+            S[idx] = (wv & 15) | ((chain + 1) << SH::LSH) | (rr.y << ELP_CSHIFT);
+            S[SH::OFSW + idx] = rr.z;
+        });
     Anchors<1> an;
     uint32_t gq, sel;
     {
@@ -933,31 +979,6 @@ __global__ void __launch_bounds__(Slab<TX, NC, SX, SXY, C>::THREADS, 1) sweep_sl
         an.xhi[0] = j == TX / NC - 1 ? 4 * (NC - 1) : -1;
         gq = (uint32_t)(n % SH::G);
         sel = (uint32_t)(n / SH::G) * 0x11u + 0x40u;
-    }
-    auto draw_colours = [&](uint32_t t, uint2 key) {   // of step t, by one warp
-        const uint4 w = philox(make_uint4(t, 0u, (uint32_t)tid | ELP_STREAM_COLOUR, 0u), key);
-        if (tid < SH::NG)
-            reinterpret_cast<uint4*>(S + SH::COLW + 4 * SH::NG * (t & 1))[tid] =
-                make_uint4(4 * bounded(w.x, NC), 4 * bounded(w.y, NC), 4 * bounded(w.z, NC), 4 * bounded(w.w, NC));
-    };
-    const BatchJob& J = a.jobs[a.items[blockIdx.x / C].x];
-    uint32_t* lat = J.lat;
-    uint32_t* rec = J.rec;
-    const uint2 key = make_uint2(J.seed, J.salt);
-    const uint32_t t0 = J.step0 + a.step_base + (a.step_dev ? *a.step_dev : 0u);
-    for (int i = tid; i < SH::R * SH::PLANES; i += SH::THREADS) {
-        const int zp = i / SH::R, xy = i % SH::R;
-        int z = SH::ZS * (int)rank + zp - SH::HALO;
-        z += z < 0 ? TX : 0; z -= z >= TX ? TX : 0;
-        const int idx = xy % TX + SX * (xy / TX) + SXY * zp;
-        uint32_t wv = __ldcg(lat + xy + SH::R * z);
-        if (wv & ELP_LBIT) {
-            const uint32_t chain = wv >> 5;
-            const uint4 rr = __ldcg(reinterpret_cast<const uint4*>(rec + ELP_REC_WORDS * (size_t)chain));
-            wv = (wv & 15) | ((chain + 1) << SH::LSH) | (rr.y << ELP_CSHIFT);
-            S[SH::OFSW + idx] = rr.z;
-        }
-        S[idx] = wv;
     }
     if (tid < 32) draw_colours(t0, key);
     uint32_t rw = own_bytes(t0, 0, gq, sel, key);
