@@ -179,9 +179,7 @@ int sum_bond(uint32_t a, uint32_t b, uint32_t* c)
     *c = ((a | b) == 0xf) ? (a & b) : (a | b);
     return elp_valid_bond(*c);
 }
-}  // namespace
-
-void elp_build_table(uint8_t tab[4096])
+void build_table(uint8_t tab[4096])
 {
     TableBuilder T;
     memset(&T, 0, sizeof(T));
@@ -232,6 +230,18 @@ void elp_build_table(uint8_t tab[4096])
     for (int row = 0; row < 256; row++)
         while (T.cnt[row] < 16) T.add((uint32_t)row / 16, (uint32_t)row % 16, 0, 0);
     for (int i = 0; i < 4096; i++) tab[i] = (uint8_t)(T.e[i] & 0xff);
+}
+}  // namespace
+
+// The steps take 20 us, and a group's move table needs the result again: built
+// once in the process.
+void elp_build_table(uint8_t tab[4096])
+{
+    static const struct Table {
+        uint8_t e[4096];
+        Table() { build_table(e); }
+    } T;
+    memcpy(tab, T.e, sizeof(T.e));
 }
 
 // Tables of the specialised sweep kernels (elp_sweep2.cu), in the order they
