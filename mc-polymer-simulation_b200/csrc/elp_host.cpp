@@ -264,8 +264,6 @@ void elp_build_table(uint8_t tab[4096])
 // the row an empty one (3) for b = 0xf (slot 1 at the last run of a linear
 // chain, which has no next run), for the 27 boundary classes (cx + 3 cy + 9 cz; 0 first plane, 1 inside, 2 last) of
 // a whole box, else once, followed by the plain word offsets.
-//
-// Then per entry the change of the anchor's word (run length and b_out).
 int elp_move_table(const elp_geometry* g, const elp_smem_layout* lay, uint32_t out[ELP_MOVES_MAX])
 {
     uint8_t tab[4096];
@@ -298,11 +296,6 @@ int elp_move_table(const elp_geometry* g, const elp_smem_layout* lay, uint32_t o
         }
     if (!g->periodic)
         for (uint32_t b = 0; b < 16; b++) out[n++] = (uint32_t)(elp_bt(b) + sx * elp_bu(b) + sxy * elp_bv(b));
-    for (uint32_t i = 0; i < ELP_MOVE_ENTRIES; i++) {
-        const uint32_t s1 = i >> 8, s2 = (i >> 4) & 15, E = out[i];
-        // the anchor's b_out before the move: s1, or (slot 0) s2
-        out[n++] = E ? ((E >> 5) & 15) - (s1 ? s1 : s2) + (E & 0x30000u) - ELP_CUNIT : 0u;
-    }
     return n;
 }
 

@@ -69,11 +69,10 @@ int elp_geometry_ok(const elp_geometry* g);
 void elp_layout(const elp_geometry* g, elp_smem_layout* lay);
 void elp_philox_host(const uint32_t ctr[4], const uint32_t key[2], uint32_t out[4]);
 void elp_build_table(uint8_t tab[4096]);
-// Move table (rows s1 = 0 .. 14), neighbour offsets (27 * 16 words for a
-// whole box, 16 + 16 for tiles) and changes of the anchor's word of the
-// specialised kernels.
+// Move table (rows s1 = 0 .. 14) and neighbour offsets (27 * 16 words for a
+// whole box, 16 + 16 for tiles) of the specialised kernels.
 #define ELP_MOVE_ENTRIES (15 * 256)
-#define ELP_MOVES_MAX (2 * ELP_MOVE_ENTRIES + 27 * 16)
+#define ELP_MOVES_MAX (ELP_MOVE_ENTRIES + 27 * 16)
 int elp_move_table(const elp_geometry* g, const elp_smem_layout* lay, uint32_t out[ELP_MOVES_MAX]);
 int elp_get_npol(double density, int N, long sites);
 // The grid of CreatePolymers (cpupol/efpol_init.c:239-283): chain p starts at

@@ -136,24 +136,14 @@ struct Shape {
     // Random bytes, one word (four substeps) per anchor and group.  With one
     // anchor a thread, and where MINB CTAs still fit on an SM (228 KB, 1 KB
     // reserved per CTA), all NG groups of the step, drawn before its substeps
-    // (PRE): no warp is late at a barrier for drawing (rings of L = 16 in
-    // sweep_box: 10.4 -> 9.9 us per step, L = 24: 19.3 -> 18.8).  Else one group's, read into registers
-    // as the group starts and overwritten with the next group's after its
-    // first barrier: with two anchors a thread the SM is full anyway (drawn
-    // ahead, L = 32 took 30.3 against 29.5, 48x24x24 tiles at L = 192 65.5
-    // against 62.8).
-    static constexpr bool fits(int words) { return (size_t)MINB * ((size_t)words * 4 + 1024) <= 233472; }
-    static constexpr bool PRE = K == 1 && fits(RNDW + NG * A);
-    // One CTA of one anchor a thread per SM is bound by latency: a second table
-    // with each entry's change of the anchor's word takes four instructions
-    // out of the move (rings of L = 24 in sweep_box: 20.2 -> 19.3 us per step,
-    // L = 72: 22.3 -> 21.7).
-    // Its loads' bank conflicts cost more where the SM is full (L = 32: 29.5
-    // against 30.4, L = 128: 18.2 against 18.4, 48x24x24 tiles at L = 192:
-    // 62.8 against 66.3).
-    static constexpr int DTABW = RNDW + (PRE ? NG : 1) * A;
-    static constexpr bool DT = K == 1 && MINB == 1 && fits(DTABW + ELP_MOVE_ENTRIES);
-    static constexpr int TOTW = DTABW + (DT ? ELP_MOVE_ENTRIES : 0);
+    // (PRE): no warp is late at a barrier for drawing (us per step: linear chains
+    // of L = 16 13.3 -> 12.9, tiles of 16^3 at L = 64 12.7 -> 12.0, 32x16x16 at
+    // L = 128 18.6 -> 17.4, 24^3 at L = 72 23.4 -> 22.5).  Else one group's, read
+    // into registers as the group starts and overwritten with the next group's
+    // after its first barrier: with two anchors a thread it makes no difference
+    // where they fit (L = 32 28.9 both ways).
+    static constexpr bool PRE = K == 1 && (size_t)MINB * ((size_t)(RNDW + NG * A) * 4 + 1024) <= 233472;
+    static constexpr int TOTW = RNDW + (PRE ? NG : 1) * A;
     static constexpr size_t BYTES = (size_t)TOTW * 4;
     // neighbour offsets in words fit 16 signed bits (else they are taken
     // modulo 2^16, the reach of a shared-memory word index)
@@ -467,6 +457,9 @@ __device__ __noinline__ uint32_t general_substeps(const Anchors<K> an, const uin
 // every other cycle) and by the chain of shared-memory loads, so the move is
 // written for few instructions: 43 per warp and substep, 21 of them on the
 // ALU pipe (the move of elp_device.cuh laid out the same way: 81 and 40).
+// (A second table with each entry's change of the anchor's word takes four of
+// them out, but its load costs as much: linear chains of L = 24 23.7 us per step
+// with it, 23.1 without, L = 40 23.6 and 23.1, L = 32 in slabs 16.0 and 15.9.)
 // One 32-bit entry of the move table carries everything the move's rows
 // decide (target, test, the new words' parts), new words come from additions,
 // and the target and next run are stored ahead of the anchor so that a move
@@ -504,7 +497,7 @@ __device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, cons
         const uint32_t w1 = SW(pB[q]);
         wB[q] = (R[q] & 0x8000u) ? w1 : wP[q];
     }
-    uint32_t E[K], D[K];
+    uint32_t E[K];
     bool c2[K];
 #pragma unroll
     for (int q = 0; q < K; q++) {
@@ -515,7 +508,6 @@ __device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, cons
         uint32_t ix = R[q] & (V[q] | 0x3Cu);
         if (c2[q] != s) ix += (wB[q] & 15) << 6;
         E[q] = SW(TAB4 + (int)ix);
-        if (SH::DT) D[q] = SW(4 * SH::DTABW + (int)ix);
     }
     int pY[K];
     uint32_t wY[K];
@@ -534,8 +526,7 @@ __device__ __forceinline__ uint32_t substepK(const Anchors<K>& an, int sh4, cons
     for (int q = 0; q < K; q++) {
         const bool s = (R[q] & 0x8000u) != 0;
         const bool ok = E[q] != 0 && (wY[q] & E[q] & (PER ? 0xFu : 0x1Fu)) == 0;
-        const uint32_t nP = SH::DT ? wP[q] + D[q]
-                                   : ((wP[q] & ~15u) | ((E[q] >> 5) & 15u)) + (E[q] & 0x30000u) - ELP_CUNIT;
+        const uint32_t nP = ((wP[q] & ~15u) | ((E[q] >> 5) & 15u)) + (E[q] & 0x30000u) - ELP_CUNIT;
         const uint32_t nB = c2[q] ? wB[q] - ELP_CUNIT : 0u;
         const uint32_t nY = wY[q] + ELP_CUNIT + ((E[q] >> 9) & 15u);
         if (ok) SW(pY[q]) = nY;
@@ -631,17 +622,14 @@ __device__ __forceinline__ void count_accepted(unsigned long long* acc, unsigned
     if ((threadIdx.x & 31) == 0 && v) atomicAdd(acc, v);
 }
 
-// Tables of a launch into shared memory: moves, neighbour offsets, changes of
-// the anchor's word (elp_move_table builds them in this order) and rows (0xf, x) of the
-// transition table (moves of a linear chain's monomer 0).
+// Tables of a launch into shared memory: moves, neighbour offsets (elp_move_table
+// builds them in this order) and rows (0xf, x) of the transition table (moves of
+// a linear chain's monomer 0).
 template <class SH, bool PER>
 __device__ __forceinline__ void load_tables(const BatchLaunch& a)
 {
-    static_assert(SH::TABS % 4 == 0 && SH::TABW % 4 == 0 && SH::DTABW % 4 == 0, "16-byte copies");
+    static_assert(SH::TABS % 4 == 0 && SH::TABW % 4 == 0, "16-byte copies");
     for (int i = threadIdx.x; i < SH::TABS / 4; i += SH::THREADS) cp_async16(g_smem + SH::TABW + 4 * i, a.moves + 4 * i);
-    if (SH::DT)
-        for (int i = threadIdx.x; i < ELP_MOVE_ENTRIES / 4; i += SH::THREADS)
-            cp_async16(g_smem + SH::DTABW + 4 * i, a.moves + SH::TABS + 4 * i);
     for (int i = threadIdx.x; i < 64; i += SH::THREADS) g_smem[SH::HTABW + i] = a.table[960 + i];
 }
 
@@ -810,8 +798,7 @@ struct Slab {
     static constexpr int TABW = (SXY * PLANES + 3) & ~3;
     static constexpr int OFFW = TABW + ELP_MOVE_ENTRIES;
     static constexpr int TABS = ELP_MOVE_ENTRIES + 27 * 16;
-    static constexpr int DTABW = TABW + TABS;
-    static constexpr int OFSW = DTABW + ELP_MOVE_ENTRIES;   // offsets by site
+    static constexpr int OFSW = TABW + TABS;                // offsets by site
     static constexpr int COLW = OFSW + TABW;                // colours of a step and the next
     static constexpr int BARW = COLW + 8 * NG;              // two mbarriers
     static constexpr size_t BYTES = (size_t)(BARW + 4) * 4;
@@ -871,12 +858,13 @@ __device__ __forceinline__ uint32_t slab_substep(const Anchors<1>& an, uint32_t 
     const bool c2 = wB >= 2u * ELP_CUNIT;
     uint32_t ix = R & (V | 0x3Cu);
     if (c2 != s) ix += (wB & 15) << 6;
-    const uint32_t E = SW(4 * SH::TABW + (int)ix), D = SW(4 * SH::DTABW + (int)ix);
+    const uint32_t E = SW(4 * SH::TABW + (int)ix);
     const uint32_t V2 = SW(tc + (int)(E >> 26));
     const int pY = p + ((int)V2 >> 14);
     const uint32_t wY = SW(pY), oY = SW(4 * SH::OFSW + pY);
     const bool ok = E != 0 && (wY & E & 0xFu) == 0, away = (E >> 28) != 0;   // away: not into the anchor's run
-    uint32_t nP = wP + D, nB = c2 ? wB - ELP_CUNIT : 0u, nY = wY + ELP_CUNIT + ((E >> 9) & 15u);
+    uint32_t nP = ((wP & ~15u) | ((E >> 5) & 15u)) + (E & 0x30000u) - ELP_CUNIT;
+    uint32_t nB = c2 ? wB - ELP_CUNIT : 0u, nY = wY + ELP_CUNIT + ((E >> 9) & 15u);
     int at = -1;                              // the run with monomer 0 whose offset changes
     uint32_t off = 0;
     if (ok && ((wB | wY) & SH::LMASK)) {
@@ -938,8 +926,6 @@ __global__ void __launch_bounds__(Slab<TX, NC, SX, SXY, C>::THREADS, 1) sweep_sl
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = tid; i < SH::TABS / 4; i += SH::THREADS) cp_async16(S + SH::TABW + 4 * i, a.moves + 4 * i);
-    for (int i = tid; i < ELP_MOVE_ENTRIES / 4; i += SH::THREADS)
-        cp_async16(S + SH::DTABW + 4 * i, a.moves + SH::TABS + 4 * i);
     auto draw_colours = [&](uint32_t t, uint2 key) {   // of step t, by one warp
         const uint4 w = philox(make_uint4(t, 0u, (uint32_t)tid | ELP_STREAM_COLOUR, 0u), key);
         if (tid < SH::NG)
