@@ -97,7 +97,7 @@ extern "C" elp_status elp_create(const elp_job_spec* spec, elp_ctx** out)
                                         error_flags(c), c->stream);
         if (eg == cudaSuccess) {
             c->group_ready = 1;
-            c->G.alone = 1;
+            c->G.sole = 1;
             elp_group_add(&c->G, c->d_lat, c->d_rec, c->d_acc, c->N, c->P, c->seed, c->salt, 0, c->linear);
             eg = elp_group_commit(&c->G);
         }

@@ -180,7 +180,7 @@ extern "C" elp_status elp_batch_create(const elp_job_spec* specs, int32_t njobs,
         elp_group_add(G, mm.lat, mm.rec, mm.acc, mm.N, mm.P, mm.seed, mm.salt, 0, mm.linear);
     }
     for (elp_group* G : b->groups) {
-        G->alone = b->groups.size() == 1;
+        G->sole = b->groups.size() == 1;
         if ((e = elp_group_commit(G)) != cudaSuccess) {
             elp_batch_destroy(b);
             return elp_fail(ELP_ERR_CUDA, "group commit failed: %s", cudaGetErrorString(e));

@@ -20,7 +20,7 @@ Sweep2Launch make_launch(const elp_group* G, int nsteps, uint32_t step_base, int
     l.sxy = G->lay.sxy;
     l.nsm = G->nsm;
     l.check_only = check_only;
-    l.alone = G->alone;
+    l.sole = G->sole;
     double sites = (double)G->g.tx * G->g.ty * G->g.tz, box = (double)G->g.L * G->g.L * G->g.L;
     for (const BatchJob& j : G->jobs) {
         double m = j.nchains * sites / box;

@@ -22,7 +22,9 @@ struct elp_group {
     int threads;                      // block size of the sweep kernel in use
     size_t smem;                      // its dynamic shared memory per block
     int spl;                          // steps per launch (tiled: specialised kernel only)
-    int alone = 0;                    // set before commit: no other group's work runs beside this one's
+    // set before commit: its context or batch has no other group.  What other
+    // contexts, batches or processes run on the device is not known here.
+    int sole = 0;
     int use_graph;                    // tiled domains: replay launches from a CUDA graph
     int graph_steps;                  // steps captured per graph (rounded down to whole launches)
     cudaStream_t stream;

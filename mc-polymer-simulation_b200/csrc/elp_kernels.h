@@ -68,7 +68,7 @@ struct Sweep2Launch {
     BatchLaunch args;
     int threads_out;               // check_only: block size of the kernel that fits
     size_t smem_out;               // check_only: its dynamic shared memory
-    int alone;                     // 1: no other group's work shares the device with this one
+    int sole;                      // 1: the only group of its context or batch
     int linear;                    // 1: some job holds linear chains (kernel with monomer-0 moves)
 };
 

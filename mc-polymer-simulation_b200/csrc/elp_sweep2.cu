@@ -1361,19 +1361,26 @@ cudaError_t launch2(const Sweep2Launch* l, Kernel k, std::atomic<int>* per_sm, c
         // 108.9 -> 106.1), where two launches' CTAs fit side by side or fill
         // the SMs anyway: in between, the early ones share an SM with their
         // like later on (125 tiles at L = 80: 16.4 -> 19.0).  Not beside other
-        // groups' work, whose place they would take while they wait.
+        // groups of a batch or a server, whose place they would take while they
+        // wait.  Other contexts cannot be seen from here; several of them at
+        // once (a thread each, 100 steps and a checked fetch in turn) still gain:
+        // L = 64 twice 12.3 -> 10.8 ms for 600 steps, eight times 35.5 -> 22.4,
+        // L = 128 four times 53.2 -> 37.5, against launches in plain order.
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = l->alone && (2 * grid <= l->nsm || grid > l->nsm);
+        attr[0].val.programmaticStreamSerializationAllowed = l->sole && (2 * grid <= l->nsm || grid > l->nsm);
     }
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k, l->args);
 }
 
-// Whole boxes of rings in C slabs.  Clusters only for melts that have the
-// device to themselves, and as many as are resident at once: a box on 8 SMs
-// takes half the time of one on a single SM, so beside other work it would
-// cost throughput.  cudaErrorNotSupported sends the caller to sweep_box.
+// Whole boxes of rings in C slabs.  Clusters only for the one group of a
+// context or batch, and as many as are resident at once: a box on 8 SMs takes
+// half the time of one on a single SM, so beside the other groups of a mix it
+// would cost throughput.  Other contexts cannot be seen from here; many at once
+// wait for the host more than for SMs (L = 32, a thread each, 600 steps and six
+// checked fetches: 8 contexts 29 ms, 40 contexts 126, on the one-SM kernel of
+// before 49 and 162).  cudaErrorNotSupported sends the caller to sweep_box.
 template <int TX, int NC, int SX, int SXY, int C>
 cudaError_t launch_slabs(const Sweep2Launch* l, cudaStream_t s)
 {
@@ -1384,7 +1391,7 @@ cudaError_t launch_slabs(const Sweep2Launch* l, cudaStream_t s)
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= MAX_DEVICES) return cudaErrorInvalidDevice;
-    if (C > 1 && !l->alone) return cudaErrorNotSupported;
+    if (C > 1 && !l->sole) return cudaErrorNotSupported;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(l->args.nitems * C));
     cfg.blockDim = dim3(SH::THREADS);
