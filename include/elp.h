@@ -82,7 +82,9 @@ void elp_default_spec(elp_job_spec* spec);
 
 /* Create a context: validates the geometry, allocates device state, uploads
  * the transition table.  The lattice starts empty (use elp_init_melt or a
- * load call). */
+ * load call).  Contexts may run side by side on a device, each from its own
+ * thread; a context does not know of others and takes the kernels that suit a
+ * melt by itself (elp_batch_* for many melts at once). */
 elp_status elp_create(const elp_job_spec* spec, elp_ctx** out);
 
 /* Reference initial melt (CreatePolymers): step counter reset to 0. */
@@ -204,7 +206,10 @@ elp_status elp_check_noalloc(const uint32_t* d_words, const uint32_t* d_records,
 #define ELP_OBS_MAX_BINS 64
 elp_status elp_observe(elp_ctx* ctx, double* cms_tuv, double* rg2, double* sl, uint64_t* run_hist, int32_t nbins);
 
-/* Raw state: words[L^3] site words, records[4*P]. Blocking. */
+/* Raw state: words[L^3] site words, records[4*P]. Blocking.  elp_set_state
+ * takes what elp_get_state gave, with edits or without; elp_check,
+ * elp_fetch_* and elp_observe take any words, elp_run only a state that
+ * elp_check passes. */
 elp_status elp_get_state(elp_ctx* ctx, uint32_t* words, uint32_t* records);
 elp_status elp_set_state(elp_ctx* ctx, const uint32_t* words, const uint32_t* records, uint64_t step);
 

@@ -739,13 +739,13 @@ __global__ void __launch_bounds__(((TX * TX * (TX / NC) / K) + 31) / 32 * 32, 1)
 // copies 26.5 us; a cluster barrier (release, acquire) per substep 20.9, as it
 // waits for every store to be acknowledged (0.31 us in a loop of its own,
 // against 0.13 for a barrier of arrivals that announce bytes); C = 4: 20.3.
-// L = 30: 28.3 -> 17.6, L = 28: 24.0 -> 14.2.  L = 26 has slabs of 13 planes
+// L = 30: 28.3 -> 18.0, L = 28: 24.0 -> 14.4.  L = 26 has slabs of 13 planes
 // only: 20.1 -> 23.0, left alone.
 //
 // The boxes that fit the threads of one CTA (up to 24^3) run as one slab: they
 // too are bound by latency, and gain from monomer 0's offsets kept by site
-// (see slab_substep).  L = 16: 9.9 -> 8.95 us per step (N = 50; N = 20: 11.2
-// -> 10.1), L = 18: 12.5 -> 11.5, L = 20: 14.4 -> 13.8, L = 22: 16.6 -> 16.3,
+// (see slab_substep).  L = 16: 9.9 -> 8.9 us per step (N = 50; N = 20: 11.2
+// -> 10.1), L = 18: 12.5 -> 11.1, L = 20: 14.4 -> 13.7, L = 22: 16.6 -> 16.0,
 // L = 24: 18.8 -> 18.6.
 __device__ __forceinline__ uint32_t cluster_address(uint32_t rank)   // of a CTA's g_smem
 {
@@ -1500,8 +1500,8 @@ extern "C" cudaError_t elp_launch_sweep2(const Sweep2Launch* l, cudaStream_t s)
 // Shapes of rings only (linear chains of these boxes are refused): the even
 // boxes between (18 to 22 as one slab, above), and the tiles that boxes of 40,
 // 60, 72, 100, 120 ... take.  On the generic kernel a step took 171 us
-// (L = 20), 175 (28), 238 (40) and 251 (72); here 13.8, 24.0 (14.2 in slabs),
-// 23.5 and 21.7.
+// (L = 20), 175 (28), 238 (40) and 251 (72); here 13.7, 24.0 (14.4 in slabs),
+// 23.1 and 22.4.
 #define TILES(X_, Y_, Z_, NC_, SX_, SXY_, CAP_, K_, MINB_)                                                       \
     if (g.tx == X_ && g.ty == Y_ && g.tz == Z_ && !g.periodic && g.ncol == NC_ && l->sx == SX_ &&                \
         l->sxy == SXY_ && !l->linear)                                                                            \

@@ -1,5 +1,6 @@
 // elp_walk.cu -- chain reconstruction and invariant kernels, for boxes too large
-// to rank (elp_rank.cu) and for the codes of melts that the ranking finds amiss.
+// to rank (elp_rank.cu), devices without room for its scratch, and the codes of
+// melts that the ranking finds amiss.
 //
 // walk_kernel rebuilds each ring (start site of monomer 0 plus N bond codes,
 // the TUV content of cpupol/efpol_io.c:70-77) from the site words by

@@ -1,7 +1,7 @@
 /*
  * elp_dump.h -- one dump of the drop-in programs: the melt's invariants are
- * checked (elp_fetch_checked: one ring walk and one site scan, efpol's codes
- * 3/4) and the TUV file is written; when the environment sets ELP_PTL=1, the
+ * checked (elp_fetch_checked: chains rebuilt and all site words added up,
+ * efpol's codes 3/4) and the TUV file is written; when the environment sets ELP_PTL=1, the
  * same state also goes out as one more line of every ring's per-ring time
  * series (SAMPLE_DIR/ptl/pol=<p>_dev=0.res, the files the reference's
  * analysis/create_ptl.c builds afterwards from the TUV dumps).  The PTL files
